@@ -18,18 +18,12 @@
 // FP32 with a cancellation-free stretch and fast intrinsics; the relative
 // comparisons util::isGreater (a - b > 1e-5 max(|a|, |b|)) become
 // comparisons against thresholds precomputed per particle.
-//
-// The state-based pre-pass (dilatation) keeps the generic tiled kernel.
-
-#include "pdgpu_bonds.cuh"
+#include "pdgpu_bulk.cuh"
+#include "pdgpu_internal.h"
 
 namespace pdgpu {
 
 namespace mixed_loop {
-
-using bonds_mixed::gmask;
-using bonds_mixed::gsum;
-using bonds_mixed::gmax;
 
 // threads per CTA: 256 in 2-D; in 3-D, where a tile's neighbour window is
 // large (~100 KB of stage) and only two CTAs fit an SM, up to 512, so that
@@ -37,49 +31,6 @@ using bonds_mixed::gmax;
 // fit the register file
 template <int DIM, int LPN>
 constexpr int kThreadsFor = DIM == 3 ? (256 * LPN < 512 ? 256 * LPN : 512) : 256;
-constexpr unsigned kWaitTries = 1u << 22;  // bounded mbarrier wait
-
-// ---- bulk copy + mbarrier (PTX) ----
-__device__ __forceinline__ uint32_t sa(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void bar_init(uint64_t *bar) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sa(bar)) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-// orders this CTA's earlier shared-memory accesses before later bulk-copy writes
-__device__ __forceinline__ void fence_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void bar_arrive_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sa(bar)), "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-          sa(dst)),
-      "l"(src), "r"(bytes), "r"(sa(bar))
-      : "memory");
-}
-__device__ __forceinline__ bool bar_try(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(sa(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// true once the phase of the given parity completed; false after kWaitTries attempts
-__device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
-  for (unsigned t = 0; t < kWaitTries; t++)
-    if (bar_try(bar, parity)) return true;
-  return false;
-}
 
 // Shared-memory plan of one tile (byte offsets into the dynamic stage);
 // identical on host and device.  Bulk-copied regions start and end on 16-byte
@@ -217,27 +168,11 @@ __device__ __forceinline__ void bond(const DevData &d, const MixParticle &M, con
   }
 }
 
-// does any bond of [b0, b1) (bit positions in the staged bitmap) start broken?
-template <int LPN>
-__device__ __forceinline__ bool any_broken(const uint32_t *s_bits, int b0, int b1, unsigned gm) {
-  const int lane = threadIdx.x % LPN;
-  const int w0 = b0 >> 5, w1 = (b1 - 1) >> 5;
-  bool hit = false;
-  for (int w = w0 + lane; w <= w1; w += LPN) {
-    uint32_t m = s_bits[w];
-    if (w == w0) m &= ~0u << (b0 & 31);
-    if (w == w1) m &= ~0u >> (31 - ((b1 - 1) & 31));
-    hit |= m != 0u;
-  }
-  return __any_sync(gm, hit);
-}
-
 template <int DIM, int LPN, int LAW, typename CT>
 __device__ __forceinline__ void tile_nodes(const DevData &d, const BondTile &T, const MixParticle &M,
                                            const View<DIM> &V, const CT *s_col, const uint32_t *s_bits,
                                            const int64_t *s_row, const Plan &p) {
   const int lane = threadIdx.x % LPN;
-  const unsigned gm = gmask<LPN>();
   const int st = DIM == 2 ? 2 : 4;
   const int64_t kb = T.bond_begin;
   const int col_off = (int)(kb - p.col0);
@@ -245,10 +180,14 @@ __device__ __forceinline__ void tile_nodes(const DevData &d, const BondTile &T, 
   const int shift = sizeof(CT) == 2 ? (int)(M.start - T.win_begin) : (int)(-T.win_begin);
   const bool gauss = d.inf.type == PDGPU_INF_GAUSSIAN;
   // every node of a tile computes forces (tiles cover force-computing particles only)
-  for (int64_t pos = T.node_begin + threadIdx.x / LPN; pos < T.node_end; pos += kThreadsFor<DIM, LPN> / LPN) {
+  // a warp's 32 / LPN nodes go through the loop together; past the tile's end
+  // a group has an empty row
+  for (int64_t wb = T.node_begin + threadIdx.x / 32 * (32 / LPN); wb < T.node_end; wb += kThreadsFor<DIM, LPN> / LPN) {
+    const int64_t pos = wb + (threadIdx.x & 31) / LPN;
+    const bool in_tile = pos < T.node_end;
     // bond scheme 2: the tile's nodes longest row first
-    const int64_t i = d.node_order ? (int64_t)d.node_order[pos] : pos;
-    const int k0 = (int)(s_row[i - p.row0] - kb), k1 = (int)(s_row[i + 1 - p.row0] - kb);
+    const int64_t i = !in_tile ? T.node_end - 1 : d.node_order ? (int64_t)d.node_order[pos] : pos;
+    const int k0 = (int)(s_row[i - p.row0] - kb), k1 = in_tile ? (int)(s_row[i + 1 - p.row0] - kb) : k0;
     const int li = (int)(i - T.win_begin);
     float xi[3], ui[3], vi;
     V.node(li, xi, ui, vi);
@@ -256,7 +195,7 @@ __device__ __forceinline__ void tile_nodes(const DevData &d, const BondTile &T, 
     if constexpr (LAW == LAW_STATE) mi = V.m[li];
     float F[3] = {0.f, 0.f, 0.f};
     float zmax = 0.f;
-    if (!any_broken<LPN>(s_bits, k0 + bit_off, k1 + bit_off, gm)) {
+    if (!any_broken<LPN>(s_bits, k0 + bit_off, k1 + bit_off)) {
       // no bond of this node starts broken: no per-bond state test; four
       // bonds in flight per thread (measured: 17 % faster than two on a
       // bond loop beyond L2, 9 % on config 1; packed FP32x2 pairs of bonds
@@ -273,11 +212,11 @@ __device__ __forceinline__ void tile_nodes(const DevData &d, const BondTile &T, 
                               kb + k, F, zmax);
       }
     }
-    const double Fx = gsum<LPN>((double)F[0], gm);
-    const double Fy = gsum<LPN>((double)F[1], gm);
-    const double Fz = DIM == 3 ? gsum<LPN>((double)F[2], gm) : 0.0;
-    const float zq = gmax<LPN>(zmax, gm);
-    if (lane == 0) {
+    const double Fx = gsum<LPN>((double)F[0]);
+    const double Fy = gsum<LPN>((double)F[1]);
+    const double Fz = DIM == 3 ? gsum<LPN>((double)F[2]) : 0.0;
+    const float zq = gmax<LPN>(zmax);
+    if (lane == 0 && in_tile) {
       d.f[st * i] = Fx;
       d.f[st * i + 1] = Fy;
       if constexpr (DIM == 3) d.f[st * i + 2] = Fz;
@@ -326,21 +265,24 @@ __device__ __forceinline__ void tile_theta(const DevData &d, const BondTile &T, 
                                            const View<DIM> &V, const CT *s_col, const uint32_t *s_bits,
                                            const int64_t *s_row, const Plan &p) {
   const int lane = threadIdx.x % LPN;
-  const unsigned gm = gmask<LPN>();
   const int64_t kb = T.bond_begin;
   const int col_off = (int)(kb - p.col0);
   const int bit_off = (int)(kb - 32 * p.word0);
   const int shift = sizeof(CT) == 2 ? (int)(M.start - T.win_begin) : (int)(-T.win_begin);
   const bool gauss = d.inf.type == PDGPU_INF_GAUSSIAN;
-  for (int64_t pos = T.node_begin + threadIdx.x / LPN; pos < T.node_end; pos += kThreadsFor<DIM, LPN> / LPN) {
+  // a warp's 32 / LPN nodes go through the loop together; past the tile's end
+  // a group has an empty row
+  for (int64_t wb = T.node_begin + threadIdx.x / 32 * (32 / LPN); wb < T.node_end; wb += kThreadsFor<DIM, LPN> / LPN) {
+    const int64_t pos = wb + (threadIdx.x & 31) / LPN;
+    const bool in_tile = pos < T.node_end;
     // bond scheme 2: the tile's nodes longest row first
-    const int64_t i = d.node_order ? (int64_t)d.node_order[pos] : pos;
-    const int k0 = (int)(s_row[i - p.row0] - kb), k1 = (int)(s_row[i + 1 - p.row0] - kb);
+    const int64_t i = !in_tile ? T.node_end - 1 : d.node_order ? (int64_t)d.node_order[pos] : pos;
+    const int k0 = (int)(s_row[i - p.row0] - kb), k1 = in_tile ? (int)(s_row[i + 1 - p.row0] - kb) : k0;
     const int li = (int)(i - T.win_begin);
     float xi[3], ui[3], vi;
     V.node(li, xi, ui, vi);
     float th = 0.f;
-    if (!any_broken<LPN>(s_bits, k0 + bit_off, k1 + bit_off, gm)) {
+    if (!any_broken<LPN>(s_bits, k0 + bit_off, k1 + bit_off)) {
 #pragma unroll 2
       for (int k = k0 + lane; k < k1; k += LPN)
         pre_bond<DIM, true>(d, M, V, xi, ui, (int)s_col[k + col_off] + shift, false, gauss, kb + k, th);
@@ -351,8 +293,8 @@ __device__ __forceinline__ void tile_theta(const DevData &d, const BondTile &T, 
         pre_bond<DIM, false>(d, M, V, xi, ui, (int)s_col[k + col_off] + shift, broken, gauss, kb + k, th);
       }
     }
-    const double t = gsum<LPN>((double)th, gm);
-    if (lane == 0) d.theta[i] = 3.0 * t / d.mx[i];
+    const double t = gsum<LPN>((double)th);
+    if (lane == 0 && in_tile) d.theta[i] = 3.0 * t / d.mx[i];
   }
 }
 
@@ -479,7 +421,6 @@ __device__ __forceinline__ void tile_sym(const DevData &d, const BondTile &T, co
                                          unsigned char *smem) {
   constexpr int kT = kThreadsFor<2, LPN>;
   const int lane = threadIdx.x % LPN;
-  const unsigned gm = gmask<LPN>();
   const int64_t kb = T.bond_begin;
   const int col_off = (int)(kb - p.col0);
   const int bit_off = (int)(kb - 32 * p.word0);
@@ -491,11 +432,14 @@ __device__ __forceinline__ void tile_sym(const DevData &d, const BondTile &T, co
   float2 *s_fj = reinterpret_cast<float2 *>(smem + q.off_fj);
   float *s_zq = reinterpret_cast<float *>(smem + q.off_zq);
   // phase A: bonds to later tile nodes and bonds leaving the tile
-  for (int64_t i = T.node_begin + threadIdx.x / LPN; i < T.node_end; i += kT / LPN) {
+  for (int64_t wb = T.node_begin + threadIdx.x / 32 * (32 / LPN); wb < T.node_end; wb += kT / LPN) {
+    const int64_t i_raw = wb + (threadIdx.x & 31) / LPN;
+    const bool in_tile = i_raw < T.node_end;
+    const int64_t i = in_tile ? i_raw : T.node_end - 1;
     const int64_t row_i = s_row[i - p.row0];
-    const int k0 = (int)(row_i - kb), k1 = (int)(s_row[i + 1 - p.row0] - kb);
+    const int k0 = (int)(row_i - kb), k1 = in_tile ? (int)(s_row[i + 1 - p.row0] - kb) : k0;
     const uint2 meta = s_meta[i - q.meta0];
-    const int base = (int)meta.x, n_up = (int)(meta.y & 0xffffu), n_uo = (int)(meta.y >> 16);
+    const int base = (int)meta.x, n_up = (int)(meta.y & 0xffffu), n_uo = in_tile ? (int)(meta.y >> 16) : 0;
     const int li = (int)(i - T.win_begin);
     float xi[3], ui[3], vi;
     V.node(li, xi, ui, vi);
@@ -503,7 +447,7 @@ __device__ __forceinline__ void tile_sym(const DevData &d, const BondTile &T, co
     if constexpr (LAW == LAW_STATE) mi = V.m[li];
     float F[3] = {0.f, 0.f, 0.f};
     float zmax = 0.f;
-    if (!any_broken<LPN>(s_bits, k0 + bit_off, k1 + bit_off, gm)) {
+    if (!any_broken<LPN>(s_bits, k0 + bit_off, k1 + bit_off)) {
 #pragma unroll 4
       for (int k = k0 + lane; k < k0 + n_uo; k += LPN)
         bond_sym<LAW, true>(d, M, V, xi, ui, vi, mi, (int)s_col[k + col_off] + shift, false, gauss, kb + k,
@@ -516,19 +460,22 @@ __device__ __forceinline__ void tile_sym(const DevData &d, const BondTile &T, co
                              row_i, i, T.win_begin, k - k0 < n_up ? base + k - k0 : -1, s_fj, s_zq, F, zmax);
       }
     }
-    const double Fx = gsum<LPN>((double)F[0], gm);
-    const double Fy = gsum<LPN>((double)F[1], gm);
-    const float zq = gmax<LPN>(zmax, gm);
-    if (lane == 0) {
+    const double Fx = gsum<LPN>((double)F[0]);
+    const double Fy = gsum<LPN>((double)F[1]);
+    const float zq = gmax<LPN>(zmax);
+    if (lane == 0 && in_tile) {
       s_pf[i - T.node_begin] = make_double2(Fx, Fy);
       s_pz[i - T.node_begin] = zq;
     }
   }
   __syncthreads();
   // phase B: the shares earlier tile nodes left for this node
-  for (int64_t i = T.node_begin + threadIdx.x / LPN; i < T.node_end; i += kT / LPN) {
-    const int k0 = (int)(s_row[i - p.row0] - kb), k1 = (int)(s_row[i + 1 - p.row0] - kb);
-    const int n_uo = (int)(s_meta[i - q.meta0].y >> 16);
+  for (int64_t wb = T.node_begin + threadIdx.x / 32 * (32 / LPN); wb < T.node_end; wb += kT / LPN) {
+    const int64_t i_raw = wb + (threadIdx.x & 31) / LPN;
+    const bool in_tile = i_raw < T.node_end;
+    const int64_t i = in_tile ? i_raw : T.node_end - 1;
+    const int k0 = (int)(s_row[i - p.row0] - kb), k1 = in_tile ? (int)(s_row[i + 1 - p.row0] - kb) : k0;
+    const int n_uo = in_tile ? (int)(s_meta[i - q.meta0].y >> 16) : 0;
     float fx = 0.f, fy = 0.f, zmax = 0.f;
 #pragma unroll 4
     for (int k = k0 + n_uo + lane; k < k1; k += LPN) {
@@ -538,10 +485,10 @@ __device__ __forceinline__ void tile_sym(const DevData &d, const BondTile &T, co
       fy += f.y;
       zmax = fmaxf(zmax, s_zq[slot]);
     }
-    const double Bx = gsum<LPN>((double)fx, gm);
-    const double By = gsum<LPN>((double)fy, gm);
-    const float zb = gmax<LPN>(zmax, gm);
-    if (lane == 0) {
+    const double Bx = gsum<LPN>((double)fx);
+    const double By = gsum<LPN>((double)fy);
+    const float zb = gmax<LPN>(zmax);
+    if (lane == 0 && in_tile) {
       const double2 a = s_pf[i - T.node_begin];
       d.f[2 * i] = a.x + Bx;
       d.f[2 * i + 1] = a.y + By;
@@ -743,19 +690,6 @@ void launch_dim(const DevData &d, const CT *col, const BondTile *t, const int *l
   }
 }
 
-template <int DIM>
-void launch_pre(const DevData &d, const BondTile *t, int n, int lanes, size_t smem, cudaStream_t s) {
-  using namespace bonds_mixed;
-  switch (lanes) {
-    case 1: k_prepass_tiled<DIM, 1><<<n, kTileThreads, smem, s>>>(d, t); break;
-    case 2: k_prepass_tiled<DIM, 2><<<n, kTileThreads, smem, s>>>(d, t); break;
-    case 4: k_prepass_tiled<DIM, 4><<<n, kTileThreads, smem, s>>>(d, t); break;
-    case 8: k_prepass_tiled<DIM, 8><<<n, kTileThreads, smem, s>>>(d, t); break;
-    case 16: k_prepass_tiled<DIM, 16><<<n, kTileThreads, smem, s>>>(d, t); break;
-    default: k_prepass_tiled<DIM, 32><<<n, kTileThreads, smem, s>>>(d, t); break;
-  }
-}
-
 template <int DIM, int LAW, typename CT, bool PRE = false, bool SYM = false>
 bool set_law_limit(size_t bytes) {
   const void *fs[] = {(const void *)k_bonds_mixed<DIM, 1, LAW, CT, PRE, SYM>,
@@ -772,13 +706,6 @@ bool set_law_limit(size_t bytes) {
 
 template <int DIM>
 int set_limit(size_t bytes) {
-  using bonds_mixed::k_prepass_tiled;
-  const void *fs[] = {(const void *)k_prepass_tiled<DIM, 1>, (const void *)k_prepass_tiled<DIM, 2>,
-                      (const void *)k_prepass_tiled<DIM, 4>, (const void *)k_prepass_tiled<DIM, 8>,
-                      (const void *)k_prepass_tiled<DIM, 16>, (const void *)k_prepass_tiled<DIM, 32>};
-  for (auto f : fs)
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-      return -1;
   const bool ok = set_law_limit<DIM, LAW_RNP, uint16_t>(bytes) && set_law_limit<DIM, LAW_PMB, uint16_t>(bytes) &&
                   set_law_limit<DIM, LAW_ELASTIC, uint16_t>(bytes) && set_law_limit<DIM, LAW_STATE, uint16_t>(bytes) &&
                   set_law_limit<DIM, LAW_RNP, int32_t>(bytes) && set_law_limit<DIM, LAW_PMB, int32_t>(bytes) &&
@@ -829,17 +756,6 @@ void launch_prepass_mixed(const DevData &d, const BondTile *t, const int *law_be
     if (d.dim == 2) launch_law<2, LAW_STATE, int32_t, true>(d, col, t + b, n, lanes, smem, s);
     else launch_law<3, LAW_STATE, int32_t, true>(d, col, t + b, n, lanes, smem, s);
   }
-}
-
-void launch_prepass_tiled_mixed(const DevData &d, const BondTile *t, int n, int lanes, size_t smem,
-                                cudaStream_t s) {
-  if (n <= 0) return;
-  if (d.dim == 2) mixed_loop::launch_pre<2>(d, t, n, lanes, smem, s);
-  else mixed_loop::launch_pre<3>(d, t, n, lanes, smem, s);
-}
-
-size_t tile_smem_mixed(int dim, bool state, int64_t window) {
-  return bonds_mixed::tile_smem_bytes(dim, state, (int)window);
 }
 
 size_t tile_smem_mixed_main(int dim, bool state, bool col16, const BondTile &t, bool sym) {

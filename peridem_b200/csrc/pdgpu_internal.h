@@ -38,6 +38,9 @@ struct DevParticle {
   double horizon, h, density, rc, kn, bound_r;
   double check_low, check_up;  // horizon -/+ 0.5 h (volume correction bounds)
   double mat[6];
+  // FP64 bond loop: reciprocals for its corrected quotients; RNP: a bond can
+  // only break where S^2 r exceeds break_q = (factor rbar)^2
+  double inv_h, inv_horizon, inv_mat3, break_q;
 };
 
 struct ContactPair {
@@ -174,6 +177,8 @@ struct DevData {
   // nodes (stride 2 doubles in 2-D, 4 in 3-D)
   double *xref, *x, *u, *v, *f;
   double *vol, *mx, *theta, *vmag;
+  double2 *fa;         // FP64 form, state-based particles: {3K/m_x - 5G/m_x, 15G/m_x}
+  double inf_inv_p1;   // 1 / inf.p1
   float *Z;
   int32_t *ptid;
   uint8_t *fix, *flags;
@@ -400,20 +405,24 @@ void launch_node_tiles(const BondTile *tiles, int n_tiles, int32_t *node_tile, c
 void launch_sym_bits(const DevData &d, const BondTile *tiles, const int32_t *node_tile, cudaStream_t s);
 void launch_tile_windows(const DevData &d, BondTile *tiles, int n_tiles, cudaStream_t s);
 // tiled bond loop (pdgpu_bonds_fp64.cu / pdgpu_bonds_mixed.cu)
-void launch_pd_tiled_fp64(const DevData &d, const BondTile *tiles, int n_tiles, int lanes,
+// law_begin[m] .. law_begin[m + 1]: the tiles of material law m (PDGPU_MAT_*);
+// stage: what of a tile sits in shared memory beside its window (bit mask of
+// the FP64 form: 1 state-law node factors, 2 dilatations, 4 bond data)
+constexpr int kStageLevels = 4;
+constexpr int kStage64[kStageLevels] = {7, 6, 4, 0};
+void launch_fp64_setup(const DevData &d, cudaStream_t s);  // node constants of the FP64 form
+// *outside = 1 if a reference distance needs the range-checked root
+void launch_fp64_range(const DevData &d, int32_t *outside, cudaStream_t s);
+void launch_pd_tiled_fp64(const DevData &d, const BondTile *tiles, const int *law_begin, int lanes, int stage,
                           size_t smem, cudaStream_t s);
-void launch_prepass_tiled_fp64(const DevData &d, const BondTile *tiles, int n_tiles, int lanes,
+void launch_prepass_tiled_fp64(const DevData &d, const BondTile *tiles, const int *law_begin, int lanes, int stage,
                                size_t smem, cudaStream_t s);
-// law_begin[m] .. law_begin[m + 1]: the tiles of material law m (PDGPU_MAT_*)
 void launch_pd_tiled_mixed(const DevData &d, const BondTile *tiles, const int *law_begin, int lanes,
                            size_t smem, cudaStream_t s);
-void launch_prepass_tiled_mixed(const DevData &d, const BondTile *tiles, int n_tiles, int lanes,
-                                size_t smem, cudaStream_t s);
 // persistent PD state pre-pass of the mixed form over the state-based tiles
 void launch_prepass_mixed(const DevData &d, const BondTile *tiles, const int *law_begin, int lanes,
                           size_t smem, cudaStream_t s);
-size_t tile_smem_fp64(int dim, bool state, int64_t window);
-size_t tile_smem_mixed(int dim, bool state, int64_t window);       // state pre-pass
+size_t tile_smem_fp64(int dim, bool state, int stage, bool col16, const BondTile &t);
 size_t tile_smem_mixed_main(int dim, bool state, bool col16, const BondTile &t, bool sym = false);
 int set_tile_smem_limit_fp64(int dim, size_t bytes);
 int set_tile_smem_limit_mixed(int dim, size_t bytes);

@@ -72,8 +72,9 @@ struct pdgpu_ctx {
   // tiled bond loop
   BondTile *tiles = nullptr;
   int n_tiles = 0;
-  size_t tile_smem = 0, tile_smem_state = 0;  // pre-pass stage; FP64 bond loop with m_x, theta
-  size_t tile_smem_pd = 0;                     // the bond-loop launch
+  size_t tile_smem_pd = 0;                     // the bond-loop and pre-pass launches
+  int stage_level0 = 0;                        // FP64 form: first staging level tried
+  int tile_stage = 0;                          // FP64 form: what is staged beside the window
   size_t tile_smem_sym = 0;                    // the symmetric bond-loop launch (mixed, 2-D)
   int bond_scheme = 0;  // 0: per node, 1: symmetric where it applies, 2: per node longest row first
   int32_t *node_tile = nullptr;                // per node its bond tile (-1: none), symmetric form
@@ -500,12 +501,52 @@ int device_error(pdgpu_ctx *ctx) {
   }
 }
 
+// 16-bit particle-local neighbour offsets where every force-computing
+// particle's nodes fit them
+int alloc_col16(pdgpu_ctx *ctx) {
+  DevData &d = ctx->d;
+  d.use16 = 1;
+  for (const auto &P : ctx->hp)
+    if (P.compute_force && P.end - P.start > 65536) d.use16 = 0;
+  if (d.use16) TRY(dalloc(ctx, &d.pd_col16, d.n_bonds + kBondPad));
+  return PDGPU_OK;
+}
+
+// node constants of the FP64 form that follow from m_x (set again when a
+// later call changes m_x)
+int fp64_node_constants(pdgpu_ctx *ctx) {
+  launch_fp64_setup(ctx->d, ctx->stream);
+  CK(cudaGetLastError());
+  CK(cudaStreamSynchronize(ctx->stream));
+  return PDGPU_OK;
+}
+
+int prepare_fp64(pdgpu_ctx *ctx) {
+  DevData &d = ctx->d;
+  bool state = false;
+  for (const auto &P : ctx->hp) state |= P.material == PDGPU_MAT_PDSTATE && P.compute_force;
+  if (state) TRY(dalloc(ctx, &d.fa, d.n_nodes));
+  d.inf_inv_p1 = 1.0 / d.inf.p1;
+  TRY(alloc_col16(ctx));
+  launch_mixed_setup(d, ctx->stream);
+  int32_t *out;
+  TRY(dalloc(ctx, &out, 1));
+  CK(cudaMemsetAsync(out, 0, 4, ctx->stream));
+  launch_fp64_range(d, out, ctx->stream);
+  int32_t outside = 0;
+  CK(cudaMemcpyAsync(&outside, out, 4, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  dfree(ctx, out);
+  // the kernels that read the bond data from global memory check every root
+  ctx->stage_level0 = outside ? kStageLevels - 1 : 0;
+  return fp64_node_constants(ctx);
+}
+
 // FP32 constants per particle for the mixed-precision bond loop
 int prepare_mixed(pdgpu_ctx *ctx) {
   DevData &d = ctx->d;
   const int64_t N = d.n_nodes;
   std::vector<MixParticle> mp(ctx->hp.size());
-  bool fits16 = true;
   for (size_t k = 0; k < ctx->hp.size(); k++) {
     const DevParticle &P = ctx->hp[k];
     MixParticle &M = mp[k];
@@ -568,12 +609,10 @@ int prepare_mixed(pdgpu_ctx *ctx) {
       M.fsc_q = (float)(t * t);
       M.nbeta_l2e = (float)(-P.mat[1] * 1.4426950408889634);
     }
-    if (P.compute_force && P.end - P.start > 65536) fits16 = false;
   }
   TRY(dalloc(ctx, &d.mixp, mp.size()));
   CK(cudaMemcpy(d.mixp, mp.data(), mp.size() * sizeof(MixParticle), cudaMemcpyHostToDevice));
-  d.use16 = fits16 ? 1 : 0;
-  if (fits16) TRY(dalloc(ctx, &d.pd_col16, d.n_bonds + kBondPad));
+  TRY(alloc_col16(ctx));
   TRY(dalloc(ctx, &d.xv_mixed, N));
   d.inf_p0 = (float)d.inf.p0;
   d.inf_p1 = (float)d.inf.p1;
@@ -583,9 +622,6 @@ int prepare_mixed(pdgpu_ctx *ctx) {
   return PDGPU_OK;
 }
 
-// Tiles of the bond loop: every force-computing particle is cut into runs of
-// tile_nodes consecutive nodes; the device finds each tile's neighbour window
-// and the largest window fixes the shared-memory stage.
 // The learned surrogate's list of bond-loop tiles (written each step by the
 // contact rebuild kernel, read by the bond loop): kept when the surrogate is
 // set, the steps rebuild contact lists (multi-particle scenes) and one
@@ -621,15 +657,53 @@ int setup_tile_list(pdgpu_ctx *ctx) {
   return PDGPU_OK;
 }
 
+// Lanes per node and nodes per tile of the bond loop, where the caller has
+// not set them: as few lanes as keep a lane's share of a row short (fewer
+// partial sums to join, fuller last rounds of a row), and tiles of one pass of
+// the CTA, two in the 2-D FP64 form (us per launch, FP64: 2-D, 333 000 nodes,
+// 84 at 4 lanes, 99 at 8; tile of 128 / 256 nodes 84 / 88; 3-D, 75 000 sphere
+// nodes, 73 at 4 lanes, 77 at 8; FP32 form, 3-D, 200 000 sphere nodes: tile of
+// 96 / 128 / 192 nodes 81 / 76 / 94).  The FP64 form raises the lanes of a
+// scene whose tiles would leave SMs idle, to the most whose one-pass tiles
+// still fit the chip at once (a pair, 317 nodes: bond loop 21 us at 8 lanes
+// and 128-node tiles, 4.8 us at 16 and 16).  The FP32 form keeps its lanes: its
+// partial sums are FP32, so their order shows in the results.
+void choose_tiling(pdgpu_ctx *ctx) {
+  const DevData &d = ctx->d;
+  const bool mixed = d.precision == PDGPU_PREC_MIXED;
+  const double bpn = (double)d.n_bonds / (double)d.n_nodes;
+  const int lanes0 = mixed && bpn <= 48 ? 1 : 4;
+  const bool choose = ctx->pd_lanes <= 0 && ctx->tile_nodes <= 0;
+  if (ctx->pd_lanes <= 0) ctx->pd_lanes = lanes0;
+  if (choose) {
+    const int threads = d.dim == 3 ? 512 : 256;
+    const int64_t room = (int64_t)sm_count() * (d.dim == 2 ? 3 : 1);  // FP64 CTAs at once
+    int64_t active = 0;
+    for (const auto &P : ctx->hp) active += P.compute_force ? P.end - P.start : 0;
+    for (int l = 2 * lanes0; !mixed && l <= 16 && l <= bpn; l *= 2) {
+      const int64_t tn = threads / l;
+      int64_t tiles = 0;
+      for (const auto &P : ctx->hp) tiles += P.compute_force ? (P.end - P.start + tn - 1) / tn : 0;
+      if (tiles > room) break;
+      ctx->pd_lanes = l;
+    }
+    ctx->tile_nodes = threads / ctx->pd_lanes;
+    if (mixed && d.dim == 3 && lanes0 == 1) ctx->tile_nodes = 256;  // one lane: 256 threads
+    if (!mixed && d.dim == 2 && active > room * ctx->tile_nodes) ctx->tile_nodes *= 2;
+  }
+  // every thread of the CTA has a node, and at least 128 (2-D) or 96 (3-D)
+  // nodes per tile
+  if (ctx->tile_nodes <= 0) ctx->tile_nodes = std::max<int64_t>(d.dim == 2 ? 128 : 96, 256 / ctx->pd_lanes);
+}
+
+// Tiles of the bond loop: every force-computing particle is cut into runs of
+// tile_nodes consecutive nodes; the device finds each tile's neighbour window
+// and the largest window fixes the shared-memory stage.
 int prepare_tiles(pdgpu_ctx *ctx) {
   DevData &d = ctx->d;
   const bool mixed = d.precision == PDGPU_PREC_MIXED;
   const size_t limit = 227 * 1024 - 1024;  // dynamic stage; static shared memory on top
-  // default: every thread of the 256-thread CTA has a node, and at least
-  // 128 (2-D) or 96 (3-D) nodes per tile
-  const int64_t tn0 = ctx->tile_nodes > 0 ? ctx->tile_nodes
-                                          : std::max<int64_t>(d.dim == 2 ? 128 : 96, 256 / ctx->pd_lanes);
-  for (int64_t tn : {tn0, (int64_t)64, (int64_t)32, (int64_t)16}) {
+  for (int64_t tn : {ctx->tile_nodes, (int64_t)64, (int64_t)32, (int64_t)16}) {
     std::vector<BondTile> t;
     for (size_t p = 0; p < ctx->hp.size(); p++) {
       const DevParticle &P = ctx->hp[p];
@@ -663,7 +737,6 @@ int prepare_tiles(pdgpu_ctx *ctx) {
                        ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     // every tile's window must hold its own nodes and fit the stage
-    int64_t wmax = 0;
     for (auto &b : t) {
       const DevParticle &P = ctx->hp[b.particle];
       if (b.win_begin < 0 || b.win_end > d.n_nodes || b.win_begin > b.node_begin ||
@@ -674,25 +747,24 @@ int prepare_tiles(pdgpu_ctx *ctx) {
       if (b.bond_begin < 0 || b.bond_end < b.bond_begin || b.bond_end > d.n_bonds)
         return fail(ctx, PDGPU_ERR_STATE, "bond tile bonds [%lld, %lld) outside [0, %lld)",
                     (long long)b.bond_begin, (long long)b.bond_end, (long long)d.n_bonds);
-      wmax = std::max(wmax, b.win_end - b.win_begin);
     }
-    const size_t sm = mixed ? tile_smem_mixed(d.dim, false, wmax) : tile_smem_fp64(d.dim, false, wmax);
-    const size_t ss = mixed ? tile_smem_mixed(d.dim, true, wmax) : tile_smem_fp64(d.dim, true, wmax);
-    // bytes of the bond-loop launch: the FP64 form stages the window only;
-    // the mixed form also holds each tile's columns and bitmap words
-    size_t pd = ctx->state_prepass ? ss : sm;
-    if (mixed) {
+    // bytes of the largest tile; the FP64 form stages as much beside the
+    // window as fits
+    size_t pd = 0;
+    int level = mixed ? 0 : ctx->stage_level0;
+    for (;; level++) {
       pd = 0;
-      for (auto &b : t)
-        pd = std::max(pd, tile_smem_mixed_main(d.dim, ctx->hp[b.particle].material == PDGPU_MAT_PDSTATE,
-                                               d.use16 != 0, b));
+      for (auto &b : t) {
+        const bool state = ctx->hp[b.particle].material == PDGPU_MAT_PDSTATE;
+        pd = std::max(pd, mixed ? tile_smem_mixed_main(d.dim, state, d.use16 != 0, b)
+                                : tile_smem_fp64(d.dim, state, kStage64[level], d.use16 != 0, b));
+      }
+      if (pd <= limit || mixed || level + 1 == kStageLevels) break;
     }
-    const size_t need = std::max(pd, ctx->state_prepass ? sm : (size_t)0);
-    if (need > limit) continue;
-    const int rc = mixed ? set_tile_smem_limit_mixed(d.dim, need) : set_tile_smem_limit_fp64(d.dim, need);
-    if (rc != 0) return fail(ctx, PDGPU_ERR_CUDA, "cannot raise the shared-memory limit to %zu bytes", need);
-    ctx->tile_smem = sm;
-    ctx->tile_smem_state = ss;
+    if (pd > limit) continue;
+    const int rc = mixed ? set_tile_smem_limit_mixed(d.dim, pd) : set_tile_smem_limit_fp64(d.dim, pd);
+    if (rc != 0) return fail(ctx, PDGPU_ERR_CUDA, "cannot raise the shared-memory limit to %zu bytes", pd);
+    ctx->tile_stage = kStage64[level];
     ctx->tile_smem_pd = pd;
     ctx->tile_nodes = tn;
     return setup_tile_list(ctx);
@@ -848,12 +920,7 @@ int prepare(pdgpu_ctx *ctx) {
   TRY(dalloc(ctx, &d.ic_particle, ctx->hp.size()));
   if (ctx->ic_sel.size() != ctx->hp.size()) ctx->ic_sel.assign(ctx->hp.size(), 0);
   CK(cudaMemcpy(d.ic_particle, ctx->ic_sel.data(), ctx->hp.size(), cudaMemcpyHostToDevice));
-  // lanes per node from the average bonds per node (measured on B200: the
-  // FP32 form runs fastest with a thread per node at ~23 bonds per node)
-  const double bpn = N ? (double)d.n_bonds / (double)N : 0.0;
-  if (ctx->pd_lanes <= 0)
-    ctx->pd_lanes = d.precision == PDGPU_PREC_MIXED ? (bpn > 48 ? 4 : 1)
-                                                    : (bpn > 48 ? 32 : (bpn > 20 ? 8 : 4));
+  choose_tiling(ctx);
   // contact buffers
   {
     int dev = 0, sms = 0;
@@ -990,6 +1057,7 @@ int prepare(pdgpu_ctx *ctx) {
   // the state pre-pass runs when particle 0 is state-based (demModel.cpp:607-610)
   ctx->state_prepass = !ctx->hp.empty() && ctx->hp[0].material == PDGPU_MAT_PDSTATE;
   if (d.precision == PDGPU_PREC_MIXED) TRY(prepare_mixed(ctx));
+  else TRY(prepare_fp64(ctx));
   TRY(prepare_tiles(ctx));
   TRY(prepare_sym(ctx));
   TRY(prepare_order(ctx));
@@ -1011,7 +1079,7 @@ void pd_forces(pdgpu_ctx *ctx) {
       });
     else
       run(ctx, "pd_prepass", [&] {
-        launch_prepass_tiled_fp64(d, ctx->tiles, ctx->n_tiles, ctx->pd_lanes, ctx->tile_smem, s);
+        launch_prepass_tiled_fp64(d, ctx->tiles, ctx->tile_law, ctx->pd_lanes, ctx->tile_stage, ctx->tile_smem_pd, s);
       });
   }
   const size_t smem = d.use_sym ? ctx->tile_smem_sym : ctx->tile_smem_pd;
@@ -1021,7 +1089,7 @@ void pd_forces(pdgpu_ctx *ctx) {
     });
   else
     run(ctx, "pd_force", [&] {
-      launch_pd_tiled_fp64(d, ctx->tiles, ctx->n_tiles, ctx->pd_lanes, smem, s);
+      launch_pd_tiled_fp64(d, ctx->tiles, ctx->tile_law, ctx->pd_lanes, ctx->tile_stage, smem, s);
     });
 }
 
@@ -1159,11 +1227,11 @@ cudaError_t graph_step(pdgpu_ctx *ctx, const char **where) {
   // main: bond loop
   if (ctx->state_prepass) {
     if (mixed) launch_prepass_mixed(d, ctx->tiles, ctx->tile_law, ctx->pd_lanes, ctx->tile_smem_pd, s);
-    else launch_prepass_tiled_fp64(d, ctx->tiles, ctx->n_tiles, ctx->pd_lanes, ctx->tile_smem, s);
+    else launch_prepass_tiled_fp64(d, ctx->tiles, ctx->tile_law, ctx->pd_lanes, ctx->tile_stage, ctx->tile_smem_pd, s);
   }
   const size_t smem = d.use_sym ? ctx->tile_smem_sym : ctx->tile_smem_pd;
   if (mixed) launch_pd_tiled_mixed(d, ctx->tiles, ctx->tile_law, ctx->pd_lanes, smem, s);
-  else launch_pd_tiled_fp64(d, ctx->tiles, ctx->n_tiles, ctx->pd_lanes, smem, s);
+  else launch_pd_tiled_fp64(d, ctx->tiles, ctx->tile_law, ctx->pd_lanes, ctx->tile_stage, smem, s);
   if (sur) {
     *where = "surrogate join";
     e = cudaStreamWaitEvent(s, ctx->ev_sur1, 0);
@@ -1326,7 +1394,7 @@ int pdgpu_upload_nodes(pdgpu_ctx *ctx, int64_t n, const double *xref, const doub
   TRY(dalloc(ctx, &d.u, sv));
   TRY(dalloc(ctx, &d.v, sv));
   TRY(dalloc(ctx, &d.f, sv));
-  TRY(dalloc(ctx, &d.vol, n));
+  TRY(dalloc(ctx, &d.vol, n + 2));  // tail padding for the bond loop's bulk copies
   TRY(dalloc(ctx, &d.mx, n));
   TRY(dalloc(ctx, &d.theta, n));
   TRY(dalloc(ctx, &d.vmag, n));
@@ -1403,6 +1471,11 @@ int pdgpu_upload_particles(pdgpu_ctx *ctx, int64_t np, const pdgpu_particle *p) 
     P.check_up = P.horizon + 0.5 * P.h;
     P.check_low = P.horizon - 0.5 * P.h;
     for (int q = 0; q < 6; q++) P.mat[q] = p[k].mat[q];
+    P.inv_h = 1.0 / P.h;
+    P.inv_horizon = 1.0 / P.horizon;
+    P.inv_mat3 = 1.0 / P.mat[3];
+    const double fr = P.mat[4] * P.mat[2];
+    P.break_q = P.mat[4] > 0.0 ? fr * fr : -1.0;
     for (int64_t i = P.start; i < P.end; i++)
       if (ctx->ptid[i] != (int32_t)k)
         return fail(ctx, PDGPU_ERR_ARG, "node %lld: particle id %d does not match particle range %lld",
@@ -1525,7 +1598,7 @@ int pdgpu_upload_mx(pdgpu_ctx *ctx, const double *mx) {
   if (!ctx->nodes) return fail(ctx, PDGPU_ERR_STATE, "upload nodes first");
   CK(cudaMemcpy(ctx->d.mx, mx, ctx->d.n_nodes * 8, cudaMemcpyHostToDevice));
   ctx->mx = true;
-  return PDGPU_OK;
+  return ctx->prepared && ctx->d.precision == PDGPU_PREC_FP64 ? fp64_node_constants(ctx) : PDGPU_OK;
 }
 
 int pdgpu_compute_mx(pdgpu_ctx *ctx) {
@@ -1537,7 +1610,7 @@ int pdgpu_compute_mx(pdgpu_ctx *ctx) {
   CK(cudaGetLastError());
   TRY(device_error(ctx));
   ctx->mx = true;
-  return PDGPU_OK;
+  return ctx->prepared && ctx->d.precision == PDGPU_PREC_FP64 ? fp64_node_constants(ctx) : PDGPU_OK;
 }
 
 int pdgpu_add_displacement_bc(pdgpu_ctx *ctx, const pdgpu_bc_set *set, const uint8_t *psel,
