@@ -47,12 +47,11 @@ struct ContactPair {
   double rc, kn, mu, betan, kappa;
 };
 
-constexpr int kDampGroup = 4;  // particles per damping CTA, at most (static shared memory)
-
 struct DampParticle {
   double bound_r, density;
   int32_t zone, type;
   int32_t q0, q1;  // the particles of its scene (all particles outside an ensemble)
+  int64_t center;  // its centre node
 };
 
 struct Influence {
@@ -225,12 +224,6 @@ struct DevData {
   int2 *c_span;          // [c_row[i], c_row[i + 1]) of compacted node t = c_nodes[t]
   uint16_t *nzone;        // zone of each node's particle
   DampParticle *dpart;   // per particle: bounding radius, density, zone, type
-  // damping CTAs: group g holds particles damp_group[g] .. damp_group[g + 1] - 1
-  // (consecutive, one scene, at most kDampGroup); null: one particle per CTA
-  int32_t *damp_group;
-  int32_t n_damp_groups;
-  double *pcen;          // per particle, this step: {x, y, z, bounding radius, vx, vy, vz, -}
-  float4 *pcen32;        // the same centre and bounding radius in FP32 (damping pre-filter)
 
   // boundary conditions: per BC node, a run of entries applied in set order
   int32_t n_ubc_sets, n_fbc_sets;
@@ -427,6 +420,8 @@ size_t tile_smem_mixed_main(int dim, bool state, bool col16, const BondTile &t, 
 int set_tile_smem_limit_fp64(int dim, size_t bytes);
 int set_tile_smem_limit_mixed(int dim, size_t bytes);
 
+// contact node pass and particle-particle damping; then, after it, the
+// particle-wall damping
 void launch_contact_force(const DevData &d, int lanes, cudaStream_t s);
 void launch_contact_owner(const DevData &d, cudaStream_t s);
 // strain and stress at the quadrature points of linear triangles (2-D):

@@ -1117,8 +1117,7 @@ constexpr int kZonePairsSmem = 256;
 // Every load a candidate needs is issued together: the compacted node and
 // its candidate span (speculatively, before the node count arrives), then the
 // node's own data with its candidate columns, then all of each candidate's
-// data at once; the zone-pair table sits in shared memory.  The first
-// threads also gather the particle centres for the damping pass.
+// data at once; the zone-pair table sits in shared memory.
 template <int DIM, int LPN>
 __global__ void __launch_bounds__(kBlock) k_contact(DevData d) {
   __shared__ ContactPair cps[kZonePairsSmem];
@@ -1134,24 +1133,6 @@ __global__ void __launch_bounds__(kBlock) k_contact(DevData d) {
   const int err = d.ctrl->error;
   if (tab)
     for (int a = threadIdx.x; a < nz * nz; a += kBlock) cps[a] = d.contact[a];
-  {
-    // particle centres (position, velocity) of this step for the damping pass
-    for (int64_t p = (int64_t)blockIdx.x * kBlock + threadIdx.x; p < d.n_particles;
-         p += (int64_t)gridDim.x * kBlock) {
-      const int64_t c = d.particles[p].center;
-      double xc[3] = {0, 0, 0}, vc[3] = {0, 0, 0};
-      ldv<DIM>(d.x, c, xc);
-      ldv<DIM>(d.v, c, vc);
-      double *o = d.pcen + 8 * p;  // {x, y, z, bounding radius, vx, vy, vz, -}
-#pragma unroll
-      for (int q = 0; q < 3; q++) {
-        o[q] = xc[q];
-        o[4 + q] = vc[q];
-      }
-      o[3] = d.dpart[p].bound_r;
-      d.pcen32[p] = make_float4((float)xc[0], (float)xc[1], (float)xc[2], (float)o[3]);
-    }
-  }
   __syncthreads();
   const int64_t nn = err ? 0 : nn_raw;
   double crd_acc = 0.0;
@@ -1247,55 +1228,167 @@ __global__ void __launch_bounds__(kBlock) k_contact(DevData d) {
 }
 
 // ---------------------------------------------------------------------------
-// The contact node pass in one kernel, warp-cooperative (the default, one
-// lane per node): a warp takes 32 consecutive compacted nodes, whose
-// candidate rows are consecutive in the entry array, and walks their
-// entries 32 at a time, coalesced.  Each lane finds its entry's node among
-// the warp's (binary search over the row starts, held one per lane), takes
-// that node's position and velocity by shuffle, and reads only the
-// candidate's position unless the pair is inside the largest contact
-// radius.  The rare contributions are then handed, in entry order, to the
-// lane that owns the node, which adds them in the reference's order (normal
-// part, then friction part, candidate by candidate).  Results equal the
-// node pass with one lane per node.
+// Particle damping of DEMModel::computeContactForces (demModel.cpp:937-1050):
+// particle-particle through particle centres and particle-wall through the
+// condensed wall nodes; the force density is applied to all nodes of the
+// particle by the external-force pass.
+//
+// Particle-particle: one warp per particle, kBlock / 32 of them per CTA.  The
+// CTA stages the centres of kBlock particles at a time in FP32 and every warp
+// tests its particle against them with a 10 % margin over the largest reach
+// any zone pair allows (coordinates rounded to FP32 move a distance by far
+// less), so that only pairs the FP64 test can pass read FP64 data.
+//
+// It reads positions only, so its CTAs ride in the contact pass's launch: a
+// launch of its own behind the contact pass finds the SMs full of bond-loop
+// CTAs (one CTA of 128 threads and 39 KB per particle or group of four, 504 /
+// 2 002 particles: 20 / 84 us beside the bond loop; a warp per particle there,
+// 14 to 21 / 73 to 85).  In the contact launch the pass ends 3.6 / 12 us later
+// than without them, and the wall part behind it takes 2 to 3 us.
 // ---------------------------------------------------------------------------
 template <int DIM>
-__global__ void __launch_bounds__(kBlock) k_contact_warp(DevData d) {
+__device__ __forceinline__ void damp_pairs(const DevData &d, int block, ContactPair *cps) {
+  __shared__ float4 s_c[kBlock];  // {x, y, z, bounding radius}
+  __shared__ int s_range[2];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int p = block * (kBlock / 32) + warp;
+  const int nz = d.n_zones;
+  const bool tab = nz * nz <= kZonePairsSmem;
+  if (tab)
+    for (int a = threadIdx.x; a < nz * nz; a += kBlock) cps[a] = d.contact[a];
+  if (threadIdx.x < 2) {
+    // the scenes of the CTA's particles, which are consecutive
+    const int last = min((block + 1) * (kBlock / 32), d.n_particles) - 1;
+    s_range[threadIdx.x] = threadIdx.x == 0 ? d.dpart[block * (kBlock / 32)].q0 : d.dpart[last].q1;
+  }
+  DampParticle P{};
+  P.type = 1;
+  double xi[3] = {0, 0, 0}, vi[3] = {0, 0, 0};
+  if (p < d.n_particles) {
+    P = d.dpart[p];
+    ldv<DIM>(d.x, P.center, xi);
+    ldv<DIM>(d.v, P.center, vi);
+  }
+  const float fxi = (float)xi[0], fyi = (float)xi[1], fzi = (float)xi[2];
+  const double Ri = P.bound_r, vol_pi = kPi * Ri * Ri;
+  const float fr = (float)Ri, rc_f = (float)(1.01 * d.rc_max);
+  double acc[3] = {0.0, 0.0, 0.0};
+  if (__syncthreads_or(d.ctrl->error != 0)) return;
+  const int q_lo = s_range[0], q_hi = s_range[1];
+  for (int tb = q_lo; tb < q_hi; tb += kBlock) {
+    __syncthreads();  // the previous centres are no longer read
+    if (tb + (int)threadIdx.x < q_hi) {
+      const int q = tb + threadIdx.x;
+      double xq[3];
+      ldv<DIM>(d.x, d.dpart[q].center, xq);
+      s_c[threadIdx.x] = make_float4((float)xq[0], (float)xq[1], (float)xq[2], (float)d.dpart[q].bound_r);
+    }
+    __syncthreads();
+    if (P.type != 0) continue;
+#pragma unroll 4
+    for (int k = 0; k < kBlock / 32; k++) {
+      const int q = tb + lane + 32 * k;
+      if (q >= P.q1 || q < P.q0 || q == p) continue;
+      const float4 cf = s_c[lane + 32 * k];
+      const float ex = cf.x - fxi, ey = cf.y - fyi, ez = cf.z - fzi;
+      const float rm = cf.w + fr + rc_f;
+      if (ex * ex + ey * ey + ez * ez > 1.17f * rm * rm) continue;
+      const DampParticle Q = d.dpart[q];
+      if (Q.type != 0) continue;
+      double xcj[3], vcj[3];
+      ldv<DIM>(d.x, Q.center, xcj);
+      ldv<DIM>(d.v, Q.center, vcj);
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        xcj[c] -= xi[c];
+        vcj[c] -= vi[c];
+      }
+      const double Rj = Q.bound_r;
+      const double d2 = dot3<DIM>(xcj, xcj);
+      const ContactPair cp = tab ? cps[P.zone * nz + Q.zone] : d.contact[P.zone * nz + Q.zone];
+      const double reach = Rj + Ri + 1.01 * cp.rc;
+      // pairs well beyond the reach cannot pass the relative-tolerance test
+      if (d2 > 1.0625 * reach * reach) continue;
+      const double dist = sqrt(d2);
+      if (is_less(dist, reach)) {
+        const double vol_pj = kPi * Rj * Rj;
+        const double m1 = P.density * vol_pi, m2 = Q.density * vol_pj;
+        const double meq = 2. * m1 * m2 / (m1 + m2);  // util::equivalentMass
+        const double bn = cp.betan * sqrt(cp.kappa * cp.rc * meq);
+        double hat[3] = {0.0, 0.0, 0.0};
+        if (is_greater(dist, 0.))
+          for (int c = 0; c < 3; c++) hat[c] = xcj[c] / dist;
+        double vm = vcj[0] * hat[0] + vcj[1] * hat[1] + vcj[2] * hat[2];
+        if (vm > 0.) vm = 0.;
+#pragma unroll
+        for (int c = 0; c < 3; c++) acc[c] += bn * vm * hat[c] / vol_pi;
+      }
+    }
+  }
+  if (P.type != 0) return;  // uniform over the warp
+#pragma unroll
+  for (int t = 0; t < 3; t++) {
+    for (int o = 16; o > 0; o >>= 1) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
+    if (lane == 0) d.fdamp[4 * p + t] = acc[t];
+  }
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kBlock) k_damp_pairs(const __grid_constant__ DevData d) {
+  __shared__ ContactPair cps[kZonePairsSmem];
+  damp_pairs<DIM>(d, (int)blockIdx.x, cps);
+}
+
+// ---------------------------------------------------------------------------
+// The contact node pass in one kernel, warp-cooperative (the default, one
+// lane per node): a warp takes up to 32 consecutive compacted nodes, whose
+// candidate rows are consecutive in the entry array, and walks their entries
+// coalesced, kContactBatch x 32 at a time: first the distance of every entry
+// (its node's and its candidate's positions, all loads of a batch in flight),
+// then, only for groups of 32 with a pair inside the largest contact radius,
+// the forces.  There each lane finds its entry's node among the warp's (binary
+// search over the row starts, held one per lane) and takes that node's data by
+// shuffle.  The contributions are then handed, in entry order, to the lane
+// that owns the node, which adds them in the reference's order (normal part,
+// then friction part, candidate by candidate).  Results equal the node pass
+// with one lane per node.
+//
+// Bound by the latency of its dependent loads (entry, position), so it wants
+// many entries in flight: a warp takes 8 or 16 nodes instead of 32 while the
+// launch has warps left over.  Against 32 nodes per warp and one group of
+// entries at a time, beside the bond loop: 332 000 nodes 12.3 -> 5.5 us, 1.3 M
+// nodes 27 -> 14, a 24 000-node packing 9.9 -> 3.8.  Limits of 80 or 64
+// registers, for more CTAs beside the bond loop, gain nothing (spills).
+// The CTAs past the contact grid run the particle-particle damping beside it.
+// ---------------------------------------------------------------------------
+constexpr int kContactBatch = 4;
+
+template <int DIM>
+__global__ void __launch_bounds__(kBlock) k_contact_warp(const __grid_constant__ DevData d) {
   __shared__ ContactPair cps[kZonePairsSmem];
   __shared__ double scr[kBlock];
   const int l32 = threadIdx.x & 31;
   const int nz = d.n_zones;
   const bool tab = nz * nz <= kZonePairsSmem;
+  if ((int)blockIdx.x >= d.contact_grid) {
+    damp_pairs<DIM>(d, (int)blockIdx.x - d.contact_grid, cps);
+    return;
+  }
   const int64_t nn_raw = d.ctrl->c_nnodes;
   const int err = d.ctrl->error;
   if (tab)
     for (int a = threadIdx.x; a < nz * nz; a += kBlock) cps[a] = d.contact[a];
-  for (int64_t p = (int64_t)blockIdx.x * kBlock + threadIdx.x; p < d.n_particles; p += (int64_t)gridDim.x * kBlock) {
-    // particle centres (position, velocity) of this step for the damping pass
-    const int64_t c = d.particles[p].center;
-    double xc[3] = {0, 0, 0}, vc[3] = {0, 0, 0};
-    ldv<DIM>(d.x, c, xc);
-    ldv<DIM>(d.v, c, vc);
-    // record {x, y, z, bounding radius, vx, vy, vz, -}: the damping pass's
-    // pair search reads only the first 32 bytes
-    double *o = d.pcen + 8 * p;
-#pragma unroll
-    for (int q = 0; q < 3; q++) {
-      o[q] = xc[q];
-      o[4 + q] = vc[q];
-    }
-    o[3] = d.dpart[p].bound_r;
-    d.pcen32[p] = make_float4((float)xc[0], (float)xc[1], (float)xc[2], (float)o[3]);
-  }
   __syncthreads();
   const int64_t nn = err ? 0 : nn_raw;
   const double rmax = d.rc_max;
-  const int64_t nwarps = (int64_t)gridDim.x * (kBlock / 32);
+  const int64_t nwarps = (int64_t)d.contact_grid * (kBlock / 32);
+  const int npw = nn <= 8 * nwarps ? 8 : (nn <= 16 * nwarps ? 16 : 32);  // nodes per warp
   double crd_acc = 0.0;
-  for (int64_t w = ((int64_t)blockIdx.x * kBlock + threadIdx.x) >> 5; w * 32 < nn; w += nwarps) {
-    const int64_t t = w * 32 + l32;
-    const bool own = t < nn;
-    const int nval = (int)min((int64_t)32, nn - w * 32);  // lanes with a node
+  // warp w of block b takes group w * grid + b: few groups spread over the SMs
+  for (int64_t w = (int64_t)(threadIdx.x >> 5) * d.contact_grid + blockIdx.x; w * npw < nn; w += nwarps) {
+    const int64_t t = w * npw + l32;
+    const int nval = (int)min((int64_t)npw, nn - w * npw);  // lanes with a node
+    const bool own = l32 < nval;
     int32_t i = 0;
     int2 sp = make_int2(0, 0);
     double yi[3] = {0, 0, 0}, vi[3] = {0, 0, 0};
@@ -1304,43 +1397,64 @@ __global__ void __launch_bounds__(kBlock) k_contact_warp(DevData d) {
     if (own) {
       i = d.c_nodes[t];
       sp = d.c_span[t];
+    }
+    const int e0 = __shfl_sync(0xffffffffu, sp.x, 0);
+    const int e1 = __shfl_sync(0xffffffffu, sp.y, nval - 1);
+    if (own) {
       pi = d.ptid[i];
       zi = d.nzone[i];
       ldv<DIM>(d.x, i, yi);
       ldv<DIM>(d.v, i, vi);
     }
-    const int e0 = __shfl_sync(0xffffffffu, sp.x, 0);
-    const int e1 = __shfl_sync(0xffffffffu, sp.y, nval - 1);
     double fx = 0.0, fy = 0.0, fz = 0.0, crd = 0.0;
-    for (int base = e0; base < e1; base += 32) {
-      const int e = base + l32;
-      // the entry's node: the last lane whose row starts at or before e
-      int o = 0;
+    for (int base0 = e0; base0 < e1; base0 += 32 * kContactBatch) {
+      int32_t jb[kContactBatch], ib[kContactBatch];
 #pragma unroll
-      for (int step = 16; step > 0; step >>= 1) {
-        const int cnd = o + step;
-        const int st = __shfl_sync(0xffffffffu, sp.x, cnd & 31);
-        if (cnd < nval && st <= e) o = cnd;
+      for (int b = 0; b < kContactBatch; b++) {
+        const int e = base0 + 32 * b + l32;
+        jb[b] = ib[b] = 0;
+        if (e < e1) {
+          jb[b] = d.c_col[e];
+          ib[b] = d.c_own[e];
+        }
       }
-      double yo[3], vo[3];
+      double yb[kContactBatch][3];
+      unsigned near = 0;  // bit b: this lane's entry of group b is inside rmax
 #pragma unroll
-      for (int q = 0; q < 3; q++) {
-        yo[q] = __shfl_sync(0xffffffffu, yi[q], o);
-        vo[q] = __shfl_sync(0xffffffffu, vi[q], o);
+      for (int b = 0; b < kContactBatch; b++) {
+        double yo[3];
+        ldv<DIM>(d.x, ib[b], yo);
+        ldv<DIM>(d.x, jb[b], yb[b]);
+#pragma unroll
+        for (int q = 0; q < 3; q++) yb[b][q] = yb[b][q] - yo[q];
       }
-      const int32_t po = __shfl_sync(0xffffffffu, pi, o);
-      const int zo = __shfl_sync(0xffffffffu, zi, o);
-      double cxn = 0.0, cyn = 0.0, czn = 0.0, cxt = 0.0, cyt = 0.0, czt = 0.0, cr = 0.0;
-      bool contrib = false;
-      if (e < e1) {
-        const int32_t j = d.c_col[e];
-        double yj[3];
-        ldv<DIM>(d.x, j, yj);
-        double yji[3];
 #pragma unroll
-        for (int q = 0; q < 3; q++) yji[q] = yj[q] - yo[q];
-        const double R = len3<DIM>(yji);
-        if (R < rmax) {
+      for (int b = 0; b < kContactBatch; b++)
+        if (base0 + 32 * b + l32 < e1 && len3<DIM>(yb[b]) < rmax) near |= 1u << b;
+#pragma unroll
+      for (int b = 0; b < kContactBatch; b++) {
+        const bool hit = (near >> b) & 1u;
+        if (!__any_sync(0xffffffffu, hit)) continue;
+        const int e = base0 + 32 * b + l32;
+        // the entry's node: the last lane whose row starts at or before e
+        int o = 0;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1) {
+          const int cnd = o + step;
+          const int st = __shfl_sync(0xffffffffu, sp.x, cnd & 31);
+          if (cnd < nval && st <= e) o = cnd;
+        }
+        double vo[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++) vo[q] = __shfl_sync(0xffffffffu, vi[q], o);
+        const int32_t po = __shfl_sync(0xffffffffu, pi, o);
+        const int zo = __shfl_sync(0xffffffffu, zi, o);
+        double cxn = 0.0, cyn = 0.0, czn = 0.0, cxt = 0.0, cyt = 0.0, czt = 0.0, cr = 0.0;
+        bool contrib = false;
+        if (hit) {
+          const int32_t j = jb[b];
+          const double(&yji)[3] = yb[b];
+          const double R = len3<DIM>(yji);
           double vj[3];
           ldv<DIM>(d.v, j, vj);
           const double volj = d.vol[j];
@@ -1388,29 +1502,29 @@ __global__ void __launch_bounds__(kBlock) k_contact_warp(DevData d) {
             }
           }
         }
-      }
-      // hand the contributions to their nodes' lanes in entry order
-      unsigned m = __ballot_sync(0xffffffffu, contrib);
-      while (m) {
-        const int src = __ffs(m) - 1;
-        m &= m - 1;
-        const int dst = __shfl_sync(0xffffffffu, o, src);
-        const double ax = __shfl_sync(0xffffffffu, cxn, src), ay = __shfl_sync(0xffffffffu, cyn, src);
-        const double bx = __shfl_sync(0xffffffffu, cxt, src), by = __shfl_sync(0xffffffffu, cyt, src);
-        const double c = __shfl_sync(0xffffffffu, cr, src);
-        double az = 0.0, bz = 0.0;
-        if constexpr (DIM == 3) {
-          az = __shfl_sync(0xffffffffu, czn, src);
-          bz = __shfl_sync(0xffffffffu, czt, src);
-        }
-        if (l32 == dst) {
-          fx += ax;
-          fy += ay;
-          if constexpr (DIM == 3) fz += az;
-          fx += bx;
-          fy += by;
-          if constexpr (DIM == 3) fz += bz;
-          if (!(c == 0.0 && signbit(c))) crd += c;
+        // hand the contributions to their nodes' lanes in entry order
+        unsigned m = __ballot_sync(0xffffffffu, contrib);
+        while (m) {
+          const int src = __ffs(m) - 1;
+          m &= m - 1;
+          const int dst = __shfl_sync(0xffffffffu, o, src);
+          const double ax = __shfl_sync(0xffffffffu, cxn, src), ay = __shfl_sync(0xffffffffu, cyn, src);
+          const double bx = __shfl_sync(0xffffffffu, cxt, src), by = __shfl_sync(0xffffffffu, cyt, src);
+          const double c = __shfl_sync(0xffffffffu, cr, src);
+          double az = 0.0, bz = 0.0;
+          if constexpr (DIM == 3) {
+            az = __shfl_sync(0xffffffffu, czn, src);
+            bz = __shfl_sync(0xffffffffu, czt, src);
+          }
+          if (l32 == dst) {
+            fx += ax;
+            fy += ay;
+            if constexpr (DIM == 3) fz += az;
+            fx += bx;
+            fy += by;
+            if constexpr (DIM == 3) fz += bz;
+            if (!(c == 0.0 && signbit(c))) crd += c;
+          }
         }
       }
     }
@@ -1419,11 +1533,15 @@ __global__ void __launch_bounds__(kBlock) k_contact_warp(DevData d) {
         const double f[3] = {fx, fy, fz};
         stv<DIM>(d.fc, i, f);
       }
-      crd_acc += crd * d.vol[i];
+      if (crd != 0.0) crd_acc += crd * d.vol[i];
       if (d.cr_t) d.cr_t[t] = crd * d.vol[i];
     }
   }
   // deterministic per-block partial of the test wall's contact reaction
+  if (!__syncthreads_or(crd_acc != 0.0)) {
+    if (threadIdx.x == 0) d.cr_partial[blockIdx.x] = 0.0;
+    return;
+  }
   scr[threadIdx.x] = crd_acc;
   __syncthreads();
   for (int h = kBlock / 2; h > 0; h >>= 1) {
@@ -1434,132 +1552,91 @@ __global__ void __launch_bounds__(kBlock) k_contact_warp(DevData d) {
 }
 
 // ---------------------------------------------------------------------------
-// Particle damping of DEMModel::computeContactForces (demModel.cpp:937-1050):
-// particle-particle through particle centres and particle-wall through the
-// condensed wall nodes.  One block per particle; the force density is applied
-// to all nodes of the particle by k_external.
+// Particle-wall damping, after the contact pass has recorded the wall nodes:
+// one warp per particle, a particle that touches no wall leaves at once.
+// Added to the particle-particle part in fdamp.
 // ---------------------------------------------------------------------------
 constexpr int kDampBlock = 128;
-constexpr int kWallSort = 4096;
+constexpr int kWallSort = 4096;  // wall pairs of one particle, at most
+constexpr int kWallWarp = 128;   // up to here the particle's own warp orders them
 
-// One CTA per group of up to kDampGroup consecutive particles of one scene
-// (d.damp_group; one particle per CTA without it): each particle record
-// loaded in the particle-particle loop serves the whole group.  A thread
-// visits the same particles q in the same order for every member as the
-// one-particle form, and keeps a partial sum per member and component in
-// shared memory, so the sums are those of the one-particle form bit for bit.
-__global__ void __launch_bounds__(kDampBlock) k_damping(DevData d, int dim) {
+// particle p's sorted wall nodes wn[0 .. nw), each distinct node once
+template <int DIM>
+__device__ __forceinline__ void damp_wall_sum(const DevData &d, int p, const int32_t *wn, int nw) {
+  const int lane = threadIdx.x & 31, nz = d.n_zones;
+  const DampParticle P = d.dpart[p];
+  const double vol_pi = kPi * P.bound_r * P.bound_r;
+  double xc[3], vc[3], acc[3] = {0.0, 0.0, 0.0};
+  ldv<DIM>(d.x, P.center, xc);
+  ldv<DIM>(d.v, P.center, vc);
+  for (int a = lane; a < nw; a += 32) {
+    const int32_t w = wn[a];
+    if (a > 0 && wn[a - 1] == w) continue;
+    const ContactPair cp = d.contact[P.zone * nz + d.nzone[w]];
+    const double meq = P.density * vol_pi;
+    const double bn = cp.betan * sqrt(cp.kappa * cp.rc * meq);
+    double xk[3], vk[3];
+    ldv<DIM>(d.x, w, xk);
+    ldv<DIM>(d.v, w, vk);
+#pragma unroll
+    for (int t = 0; t < 3; t++) {
+      xk[t] -= xc[t];
+      vk[t] -= vc[t];
+    }
+    const double l = len3<DIM>(xk);
+    double hat[3] = {0.0, 0.0, 0.0};
+    if (is_greater(l, 0.))
+      for (int t = 0; t < 3; t++) hat[t] = xk[t] / l;
+    double vm = vk[0] * hat[0] + vk[1] * hat[1] + vk[2] * hat[2];
+    if (vm > 0.) vm = 0.;
+#pragma unroll
+    for (int t = 0; t < 3; t++) acc[t] += bn * vm * hat[t] / vol_pi;
+  }
+#pragma unroll
+  for (int t = 0; t < 3; t++) {
+    for (int o = 16; o > 0; o >>= 1) acc[t] += __shfl_xor_sync(0xffffffffu, acc[t], o);
+    if (lane == 0) d.fdamp[4 * p + t] += acc[t];
+  }
+  if (lane == 0) d.wp_cnt[p] = 0;
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(kDampBlock) k_damp_walls(const __grid_constant__ DevData d) {
   __shared__ int32_t wn[kWallSort];
-  __shared__ double red[3][kDampBlock / 32];
-  __shared__ ContactPair cps[kZonePairsSmem];
-  __shared__ double s_acc[kDampGroup][3][kDampBlock];  // member, component, thread
-  __shared__ double s_c[kDampGroup][8];                // centre (3), centre velocity (3), radius, density
-  __shared__ int s_zone[kDampGroup], s_type[kDampGroup];
-  __shared__ float4 s_cf[kDampGroup];                  // FP32 centre and radius
-  const int p0 = d.damp_group ? d.damp_group[blockIdx.x] : (int)blockIdx.x;
-  const int np = d.damp_group ? d.damp_group[blockIdx.x + 1] - p0 : 1;
-  const int nz = d.n_zones;
-  const bool tab = nz * nz <= kZonePairsSmem;
-  if (tab)
-    for (int a = threadIdx.x; a < nz * nz; a += blockDim.x) cps[a] = d.contact[a];
-  if ((int)threadIdx.x < np) {
-    const int p = p0 + threadIdx.x;
-    const DampParticle P = d.dpart[p];
-    for (int q = 0; q < 3; q++) {
-      s_c[threadIdx.x][q] = d.pcen[8 * p + q];
-      s_c[threadIdx.x][3 + q] = d.pcen[8 * p + 4 + q];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int p = blockIdx.x * (kDampBlock / 32) + warp;
+  const int cap = min(d.wp_cap, kWallSort);  // the capacity is validated on the host
+  const int nw = p < d.n_particles && !d.ctrl->error ? min(d.wp_cnt[p], cap) : 0;
+  if (nw > 0 && nw <= kWallWarp) {  // ordered by counting
+    int32_t *mine = wn + warp * (2 * kWallWarp);
+    for (int a = lane; a < nw; a += 32) mine[a] = d.wp[(int64_t)p * d.wp_cap + a];
+    __syncwarp();
+    for (int a = lane; a < nw; a += 32) {
+      const int32_t va = mine[a];
+      int rank = 0;
+      for (int b = 0; b < nw; b++) rank += mine[b] < va || (mine[b] == va && b < a);
+      mine[kWallWarp + rank] = va;
     }
-    s_c[threadIdx.x][6] = P.bound_r;
-    s_c[threadIdx.x][7] = P.density;
-    s_cf[threadIdx.x] = d.pcen32[p];
-    s_zone[threadIdx.x] = P.zone;
-    s_type[threadIdx.x] = P.type;
+    __syncwarp();
+    damp_wall_sum<DIM>(d, p, mine + kWallWarp, nw);
   }
-  for (int e = threadIdx.x; e < kDampGroup * 3 * kDampBlock; e += blockDim.x) (&s_acc[0][0][0])[e] = 0.0;
+  if (!__syncthreads_or(nw > kWallWarp)) return;
+  // more: the whole CTA sorts them, one particle after another
+  __shared__ int s_nw[kDampBlock / 32];
+  if (lane == 0) s_nw[warp] = nw;
   __syncthreads();
-  bool any = false;
-  for (int k = 0; k < np; k++) any |= s_type[k] == 0;
-  if (!any) return;
-  if (d.ctrl->error) return;
-  const DampParticle G = d.dpart[p0];  // the group's scene: its particles q0 .. q1 - 1
-  // particle-particle, over the particles of the scene: first the 16-byte
-  // FP32 {centre, radius} record, against the largest reach any zone pair
-  // allows with a 10 % margin over the FP64 test below (coordinates rounded
-  // to FP32 move a distance by far less), so that only pairs that test can
-  // pass read the FP64 record; kDampBatch records in flight per thread, each
-  // thread visiting its particles in increasing order
-  constexpr int kDampBatch = 4;
-  const float rc_f = (float)(1.01 * d.rc_max);
-  for (int qb = G.q0 + threadIdx.x; qb < G.q1; qb += kDampBatch * blockDim.x) {
-    float4 cf[kDampBatch];
-#pragma unroll
-    for (int t = 0; t < kDampBatch; t++) {
-      const int q = qb + t * (int)blockDim.x;
-      cf[t] = q < G.q1 ? d.pcen32[q] : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-#pragma unroll
-    for (int t = 0; t < kDampBatch; t++) {
-      const int q = qb + t * (int)blockDim.x;
-      if (q >= G.q1) continue;
-      for (int k = 0; k < np; k++) {
-        if (s_type[k] != 0 || q == p0 + k) continue;
-        const float4 pf = s_cf[k];
-        const float ex = cf[t].x - pf.x, ey = cf[t].y - pf.y, ez = cf[t].z - pf.z;
-        const float rm = cf[t].w + pf.w + rc_f;
-        if (ex * ex + ey * ey + ez * ez > 1.17f * rm * rm) continue;
-        const double2 c01 = *reinterpret_cast<const double2 *>(d.pcen + 8 * q);
-        const double2 c2r = *reinterpret_cast<const double2 *>(d.pcen + 8 * q + 2);
-        const double *C = s_c[k];
-        const double Ri = C[6];
-        double xcj[3] = {c01.x - C[0], c01.y - C[1], c2r.x - C[2]};
-        const double d2 = xcj[0] * xcj[0] + xcj[1] * xcj[1] + xcj[2] * xcj[2];
-        const double reach_max = c2r.y + Ri + 1.01 * d.rc_max;
-        if (d2 > 1.0625 * reach_max * reach_max) continue;
-        const DampParticle Q = d.dpart[q];
-        if (Q.type != 0) continue;
-        const double Rj = Q.bound_r;
-        double vcj[3];
-        for (int c = 0; c < 3; c++) vcj[c] = d.pcen[8 * q + 4 + c] - C[3 + c];
-        const ContactPair cp = tab ? cps[s_zone[k] * nz + Q.zone] : d.contact[s_zone[k] * nz + Q.zone];
-        const double reach = Rj + Ri + 1.01 * cp.rc;
-        // pairs well beyond the reach cannot pass the relative-tolerance test
-        if (d2 > 1.0625 * reach * reach) continue;
-        const double dist = sqrt(d2);
-        if (is_less(dist, reach)) {
-          const double vol_pi = kPi * Ri * Ri;
-          const double vol_pj = kPi * Rj * Rj;
-          const double m1 = C[7] * vol_pi, m2 = Q.density * vol_pj;
-          const double meq = 2. * m1 * m2 / (m1 + m2);  // util::equivalentMass
-          const double bn = cp.betan * sqrt(cp.kappa * cp.rc * meq);
-          double hat[3] = {0.0, 0.0, 0.0};
-          if (is_greater(dist, 0.))
-            for (int c = 0; c < 3; c++) hat[c] = xcj[c] / dist;
-          double vm = vcj[0] * hat[0] + vcj[1] * hat[1] + vcj[2] * hat[2];
-          if (vm > 0.) vm = 0.;
-          for (int c = 0; c < 3; c++) s_acc[k][c][threadIdx.x] += bn * vm * hat[c] / vol_pi;
-        }
-      }
-    }
-  }
-  // per member: particle-wall (unique wall nodes within the contact radius
-  // of any node), then the block reduction
-  const int st = dim == 2 ? 2 : 4;
-  for (int k = 0; k < np; k++) {
-    if (s_type[k] != 0) continue;  // uniform over the CTA
-    const int p = p0 + k;
-    const double *C = s_c[k];
-    const double Ri = C[6], vol_pi = kPi * Ri * Ri, rhoi = C[7];
-    int nw = d.wp_cnt[p];
-    if (nw > d.wp_cap) nw = d.wp_cap;
-    if (nw > kWallSort) nw = kWallSort;  // capacity is validated on the host
+  for (int k = 0; k < kDampBlock / 32; k++) {
+    const int n = s_nw[k];
+    if (n <= kWallWarp) continue;  // uniform over the CTA
+    const int pk = blockIdx.x * (kDampBlock / 32) + k;
     int sz = 1;
-    while (sz < nw) sz <<= 1;
-    for (int a = threadIdx.x; a < sz; a += blockDim.x)
-      wn[a] = a < nw ? d.wp[(int64_t)p * d.wp_cap + a] : INT32_MAX;
+    while (sz < n) sz <<= 1;
+    for (int a = threadIdx.x; a < sz; a += kDampBlock)
+      wn[a] = a < n ? d.wp[(int64_t)pk * d.wp_cap + a] : INT32_MAX;
     __syncthreads();
     for (int kk = 2; kk <= sz; kk <<= 1)
       for (int jj = kk >> 1; jj > 0; jj >>= 1) {
-        for (int a = threadIdx.x; a < sz; a += blockDim.x) {
+        for (int a = threadIdx.x; a < sz; a += kDampBlock) {
           const int b = a ^ jj;
           if (b > a) {
             const bool up = (a & kk) == 0;
@@ -1572,43 +1649,8 @@ __global__ void __launch_bounds__(kDampBlock) k_damping(DevData d, int dim) {
         }
         __syncthreads();
       }
-    double acc[3] = {s_acc[k][0][threadIdx.x], s_acc[k][1][threadIdx.x], s_acc[k][2][threadIdx.x]};
-    for (int a = threadIdx.x; a < nw; a += blockDim.x) {
-      const int32_t w = wn[a];
-      if (a > 0 && wn[a - 1] == w) continue;
-      const int zk = d.nzone[w];
-      const ContactPair cp = tab ? cps[s_zone[k] * nz + zk] : d.contact[s_zone[k] * nz + zk];
-      const double meq = rhoi * vol_pi;
-      const double bn = cp.betan * sqrt(cp.kappa * cp.rc * meq);
-      double xk[3] = {0, 0, 0}, vk[3] = {0, 0, 0};
-      for (int t = 0; t < dim; t++) {
-        xk[t] = d.x[st * (int64_t)w + t] - C[t];
-        vk[t] = d.v[st * (int64_t)w + t] - C[3 + t];
-      }
-      const double l = sqrt(xk[0] * xk[0] + xk[1] * xk[1] + xk[2] * xk[2]);
-      double hat[3] = {0.0, 0.0, 0.0};
-      if (is_greater(l, 0.))
-        for (int t = 0; t < 3; t++) hat[t] = xk[t] / l;
-      double vm = vk[0] * hat[0] + vk[1] * hat[1] + vk[2] * hat[2];
-      if (vm > 0.) vm = 0.;
-      for (int t = 0; t < 3; t++) acc[t] += bn * vm * hat[t] / vol_pi;
-    }
-    // block reduction (fixed order)
-    for (int t = 0; t < 3; t++) {
-      double v = acc[t];
-      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if ((threadIdx.x & 31) == 0) red[t][threadIdx.x >> 5] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (int t = 0; t < 3; t++) {
-        double s = 0.0;
-        for (int w = 0; w < kDampBlock / 32; w++) s += red[t][w];
-        d.fdamp[4 * p + t] = s;
-      }
-      d.wp_cnt[p] = 0;
-    }
-    __syncthreads();  // before wn and red are reused
+    if (warp == k) damp_wall_sum<DIM>(d, pk, wn, n);
+    __syncthreads();  // the array is free
   }
 }
 
@@ -2147,10 +2189,12 @@ void launch_contact_owner(const DevData &d, cudaStream_t s) {
 void launch_contact_force(const DevData &d, int lanes, cudaStream_t s) {
   const unsigned g = (unsigned)d.contact_grid;
   if (lanes == 1) {  // one kernel, a warp per 32 nodes
-    if (d.dim == 2) k_contact_warp<2><<<g, kBlock, 0, s>>>(d);
-    else k_contact_warp<3><<<g, kBlock, 0, s>>>(d);
+    const unsigned gc = g + blocks_for(d.n_particles, kBlock / 32);
+    if (d.dim == 2) k_contact_warp<2><<<gc, kBlock, 0, s>>>(d);
+    else k_contact_warp<3><<<gc, kBlock, 0, s>>>(d);
     return;
   }
+  PDGPU_DIM_DISPATCH(d, k_damp_pairs, <<<blocks_for(d.n_particles, kBlock / 32), kBlock, 0, s>>>(d));
   // the distance pass: eight CTAs per SM, grid-stride over the entries
   if (d.dim == 2) k_contact_near<2><<<sm_count() * 8, kBlock, 0, s>>>(d);
   else k_contact_near<3><<<sm_count() * 8, kBlock, 0, s>>>(d);
@@ -2177,7 +2221,7 @@ void launch_scene_post(const DevData &d, cudaStream_t s) {
 
 void launch_damping(const DevData &d, cudaStream_t s) {
   if (d.n_particles <= 0) return;
-  k_damping<<<d.damp_group ? d.n_damp_groups : d.n_particles, kDampBlock, 0, s>>>(d, d.dim);
+  PDGPU_DIM_DISPATCH(d, k_damp_walls, <<<blocks_for(d.n_particles, kDampBlock / 32), kDampBlock, 0, s>>>(d));
 }
 
 void launch_external(const DevData &d, cudaStream_t s) {
