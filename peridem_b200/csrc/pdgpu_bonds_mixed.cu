@@ -3,12 +3,13 @@
 //
 // One CTA per tile of one particle's nodes (the tiles of the FP64 form).
 // At the start of a tile:
-//   * one thread hands the tile's neighbour columns (16- or 32-bit) and the
-//     words of the broken-bond bitmap to the bulk-copy engine
-//     (cp.async.bulk, completion counted on an mbarrier);
-//   * all threads stage the neighbour window as packed FP32 node records
-//     (2-D: {x, y, ux, uy} + volume; 3-D: {x, y, z, volume} + {ux, uy, uz}),
-//     coordinates relative to the particle centre.
+//   * one thread hands the tile's neighbour columns (16- or 32-bit), row
+//     offsets, words of the broken-bond bitmap and the window's node records
+//     {x, y, z, volume} (relative to the particle centre) to the bulk-copy
+//     engine (cp.async.bulk, completion counted on an mbarrier), in 3-D also
+//     the displacements and the state-based law's records;
+//   * in 2-D all threads stage the window's displacements (FP64 in memory) as
+//     FP32 relative to the centre's.
 // The bond loop then reads only shared memory.  Each material law is its own
 // instantiation, so the per-bond path carries no material dispatch; every
 // index inside a tile is 32-bit.
@@ -18,6 +19,17 @@
 // FP32 with a cancellation-free stretch and fast intrinsics; the relative
 // comparisons util::isGreater (a - b > 1e-5 max(|a|, |b|)) become
 // comparisons against thresholds precomputed per particle.
+//
+// What bounds it: instruction issue (about 31 FP32 and 20 other thread
+// instructions per bond in 2-D, 57-65 % issue active) and, around it, the
+// barriers and loads at the start of each tile.  Measured per launch against
+// the loop with its break and influence tests inside, 256 threads per CTA and
+// every window node converted by its tile (B200, us, results the same to the
+// bit): 2-D RNP, 321 000 nodes, 7.2 M bonds 39 -> 26 beside the contact pass,
+// 1.26 M nodes 109 -> 82; 3-D PD state, 200 000 sphere nodes, 17.3 M bonds:
+// pre-pass 95 -> 56, main loop 78 -> 61.
+#include <cfloat>
+
 #include "pdgpu_bulk.cuh"
 #include "pdgpu_internal.h"
 
@@ -25,12 +37,14 @@ namespace pdgpu {
 
 namespace mixed_loop {
 
-// threads per CTA: 256 in 2-D; in 3-D, where a tile's neighbour window is
-// large (~100 KB of stage) and only two CTAs fit an SM, up to 512, so that
-// two CTAs per SM (one computing while the other waits at a tile barrier)
-// fit the register file
+// threads per CTA: 128 in 2-D (fewer warps to wait for one another at a
+// tile's barriers, and the last tile of a particle wastes less than with 256:
+// 332 000 nodes 28.5 us against 30.5, 1.3 M nodes 77 against 84); in 3-D, where
+// a tile's neighbour window is large (~100 KB of stage) and only two CTAs fit
+// an SM, up to 512, so that two CTAs per SM (one computing while the other
+// waits at a tile barrier) fit the register file
 template <int DIM, int LPN>
-constexpr int kThreadsFor = DIM == 3 ? (256 * LPN < 512 ? 256 * LPN : 512) : 256;
+constexpr int kThreadsFor = DIM == 3 ? (256 * LPN < 512 ? 256 * LPN : 512) : 128;
 
 // Shared-memory plan of one tile (byte offsets into the dynamic stage);
 // identical on host and device.  Bulk-copied regions start and end on 16-byte
@@ -39,12 +53,14 @@ struct Plan {
   int64_t col0;   // first column entry copied
   int64_t word0;  // first bitmap word copied
   int64_t row0;   // first row offset copied (pd_row)
-  uint32_t col_bytes, bit_bytes, row_bytes;
+  int64_t m0;     // first state record copied (8 bytes each: an even node)
+  uint32_t col_bytes, bit_bytes, row_bytes, m_bytes;
   uint32_t off_row, off_xv, off_u, off_m, total;
 };
 
 __host__ __device__ inline Plan plan(int dim, bool state, int col_size, int64_t kb, int64_t ke,
-                                     int64_t nb, int64_t ne, int64_t w) {
+                                     int64_t nb, int64_t ne, int64_t wb, int64_t we) {
+  const int64_t w = we - wb;
   Plan p;
   const int64_t per16 = 16 / col_size;
   p.col0 = kb / per16 * per16;
@@ -59,8 +75,10 @@ __host__ __device__ inline Plan plan(int dim, bool state, int col_size, int64_t 
   p.off_row = p.col_bytes + p.bit_bytes;
   p.off_xv = p.off_row + p.row_bytes;                        // float4 {x, y, z, vol}
   p.off_u = p.off_xv + (uint32_t)(16 * w);                   // 2-D float2 | 3-D float4 u
-  p.off_m = p.off_u + (uint32_t)((dim == 2 ? 8 : 16) * w);   // state: float2 per node
-  p.total = p.off_m + (state ? (uint32_t)(8 * w) : 0u);
+  p.off_m = (p.off_u + (uint32_t)((dim == 2 ? 8 : 16) * w) + 15) / 16 * 16;  // state: float2 per node
+  p.m0 = wb / 2 * 2;
+  p.m_bytes = state ? (uint32_t)(((we + 1) / 2 * 2 - p.m0) * 8) : 0u;
+  p.total = p.off_m + p.m_bytes;
   p.total = (p.total + 15) / 16 * 16;
   return p;
 }
@@ -74,6 +92,11 @@ struct View {
   const float2 *u2;  // 2-D displacement relative to the centre's
   const float4 *u4;  // 3-D displacement relative to the centre's
   const float2 *m;   // state: {theta (3K - 5G) / m_x, 15 G / m_x}
+
+  // the same records counted from node `shift` of the window
+  __device__ __forceinline__ View from(int shift) const {
+    return View{xv + shift, DIM == 2 ? u2 + shift : u2, DIM == 3 ? u4 + shift : u4, m + shift};
+  }
 
   __device__ __forceinline__ void node(int l, float (&x)[3], float (&u)[3], float &v) const {
     const float4 p = xv[l];
@@ -104,12 +127,12 @@ __device__ __forceinline__ float ex2(float x) {
 
 // One bond (i, j) of node i for one material law.  zq tracks the damage
 // measure in a monotone form: RNP S^2 r (Z = sqrt(zq) / rbar), the others
-// |S| (Z = zq / s0).  `broken` is the bond's state before this step.
-template <int DIM, int LAW, bool BROKEN_KNOWN_CLEAR>
+// |S| (Z = zq / s0).  TEST: the bond may be broken (`broken`, its state before
+// this step) or break now; without it neither is looked at.
+template <int DIM, int LAW, bool TEST, bool GAUSS>
 __device__ __forceinline__ void bond(const DevData &d, const MixParticle &M, const View<DIM> &V,
                                      const float (&xi)[3], const float (&ui)[3], float2 mi, int lj,
-                                     bool broken, bool gauss, int64_t kglob, float (&F)[3],
-                                     float &zmax) {
+                                     bool broken, int64_t kglob, float (&F)[3], float &zmax) {
   float xj[3], uj[3], volj;
   V.node(lj, xj, uj, volj);
   float dx[3], du[3], y[3];
@@ -135,18 +158,18 @@ __device__ __forceinline__ void bond(const DevData &d, const MixParticle &M, con
     zq = fabsf(S);
   }
   zmax = fmaxf(zmax, zq);
-  if (BROKEN_KNOWN_CLEAR || !broken) {
+  if (!TEST || !broken) {
     const float vol = volj * (rji > M.low_thr ? fmaf(-rji, M.inv_h, M.cu_h) : 1.f);
     // influence times the law's constant
-    const float kJ = gauss ? M.kj0 * ex2(rji * rji * M.j1) : fmaf(M.kj1, rji, M.kj0);
+    const float kJ = GAUSS ? M.kj0 * ex2(rji * rji * M.j1) : fmaf(M.kj1, rji, M.kj0);
     float sf = 0.f;
     if constexpr (LAW == LAW_RNP) {
-      if (M.irreversible && zq > M.fsc_q)
+      if (TEST && M.irreversible && zq > M.fsc_q)
         atomicOr(d.bond_bits + (kglob >> 5), 1u << (kglob & 31));
       else
         sf = kJ * S * ex2(M.nbeta_l2e * zq) * vol * inv_r;
     } else if constexpr (LAW == LAW_PMB) {
-      if (zq > M.s0_thr)
+      if (TEST && zq > M.s0_thr)
         atomicOr(d.bond_bits + (kglob >> 5), 1u << (kglob & 31));
       else
         sf = kJ * S * vol * inv_ly;
@@ -178,8 +201,11 @@ __device__ __forceinline__ void tile_nodes(const DevData &d, const BondTile &T, 
   const int col_off = (int)(kb - p.col0);
   const int bit_off = (int)(kb - 32 * p.word0);
   const int shift = sizeof(CT) == 2 ? (int)(M.start - T.win_begin) : (int)(-T.win_begin);
+  const View<DIM> N = V.from(shift);  // indexed by neighbour column
+  const CT *cols = s_col + col_off;
   const bool gauss = d.inf.type == PDGPU_INF_GAUSSIAN;
-  // every node of a tile computes forces (tiles cover force-computing particles only)
+  const float break_z = LAW == LAW_RNP ? (M.irreversible ? M.fsc_q : FLT_MAX) : (LAW == LAW_PMB ? M.s0_thr : FLT_MAX);
+  // every node of a tile computes forces (tiles cover force-computing particles only);
   // a warp's 32 / LPN nodes go through the loop together; past the tile's end
   // a group has an empty row
   for (int64_t wb = T.node_begin + threadIdx.x / 32 * (32 / LPN); wb < T.node_end; wb += kThreadsFor<DIM, LPN> / LPN) {
@@ -195,23 +221,34 @@ __device__ __forceinline__ void tile_nodes(const DevData &d, const BondTile &T, 
     if constexpr (LAW == LAW_STATE) mi = V.m[li];
     float F[3] = {0.f, 0.f, 0.f};
     float zmax = 0.f;
-    if (!any_broken<LPN>(s_bits, k0 + bit_off, k1 + bit_off)) {
-      // no bond of this node starts broken: no per-bond state test; four
-      // bonds in flight per thread (measured: 17 % faster than two on a
-      // bond loop beyond L2, 9 % on config 1; packed FP32x2 pairs of bonds
-      // measured 12 % slower on the 2-D compressive test)
+    // A node none of whose bonds starts broken is summed without any test of
+    // the bonds' states, four bonds in flight per thread (measured: 17 %
+    // faster than two on a bond loop beyond L2; packed FP32x2 pairs of bonds
+    // 12 % slower on the 2-D compressive test), and again with the tests only
+    // when its largest stretch measure breaks a bond.
+    bool test = any_broken<LPN>(s_bits, k0 + bit_off, k1 + bit_off);
+    if (!test) {
+      if (gauss) {
+#pragma unroll 2
+        for (int k = k0 + lane; k < k1; k += LPN)
+          bond<DIM, LAW, false, true>(d, M, N, xi, ui, mi, (int)cols[k], false, 0, F, zmax);
+      } else {
 #pragma unroll 4
-      for (int k = k0 + lane; k < k1; k += LPN)
-        bond<DIM, LAW, true>(d, M, V, xi, ui, mi, (int)s_col[k + col_off] + shift, false, gauss,
-                             kb + k, F, zmax);
-    } else {
+        for (int k = k0 + lane; k < k1; k += LPN)
+          bond<DIM, LAW, false, false>(d, M, N, xi, ui, mi, (int)cols[k], false, 0, F, zmax);
+      }
+    }
+    if constexpr (LAW == LAW_RNP || LAW == LAW_PMB) test |= gmax<LPN>(zmax) > break_z;
+    if (test) {
+      F[0] = F[1] = F[2] = zmax = 0.f;
       for (int k = k0 + lane; k < k1; k += LPN) {
         const int b = k + bit_off;
         const bool broken = (s_bits[b >> 5] >> (b & 31)) & 1u;
-        bond<DIM, LAW, false>(d, M, V, xi, ui, mi, (int)s_col[k + col_off] + shift, broken, gauss,
-                              kb + k, F, zmax);
+        if (gauss) bond<DIM, LAW, true, true>(d, M, N, xi, ui, mi, (int)cols[k], broken, kb + k, F, zmax);
+        else bond<DIM, LAW, true, false>(d, M, N, xi, ui, mi, (int)cols[k], broken, kb + k, F, zmax);
       }
     }
+    __syncwarp();
     const double Fx = gsum<LPN>((double)F[0]);
     const double Fy = gsum<LPN>((double)F[1]);
     const double Fz = DIM == 3 ? gsum<LPN>((double)F[2]) : 0.0;
@@ -229,10 +266,10 @@ __device__ __forceinline__ void tile_nodes(const DevData &d, const BondTile &T, 
 // e = |y| - r (cancellation-free) and, for a bond that is not broken, its
 // term r e J(r) vol_j of the dilatation sum; a bond whose stretch exceeds
 // the critical stretch breaks here (the main loop then sees it broken).
-template <int DIM, bool BROKEN_KNOWN_CLEAR>
+template <int DIM, bool TEST, bool GAUSS>
 __device__ __forceinline__ void pre_bond(const DevData &d, const MixParticle &M, const View<DIM> &V,
                                          const float (&xi)[3], const float (&ui)[3], int lj, bool broken,
-                                         bool gauss, int64_t kglob, float &th) {
+                                         int64_t kglob, float &th, float &zmax) {
   float xj[3], uj[3], volj;
   V.node(lj, xj, uj, volj);
   float dx[3], eta[3], y[3];
@@ -248,15 +285,43 @@ __device__ __forceinline__ void pre_bond(const DevData &d, const MixParticle &M,
   const float y2 = dot<DIM>(y, y);
   const float l = y2 * rsqrtf(y2);
   const float cl = __fdividef(2.f * dot<DIM>(dx, eta) + dot<DIM>(eta, eta), l + rji);
-  if (BROKEN_KNOWN_CLEAR || !broken) {
-    if (fabsf(cl * inv_r) > M.s0_thr) {
+  const float zq = fabsf(cl * inv_r);
+  zmax = fmaxf(zmax, zq);
+  if (!TEST || !broken) {
+    if (TEST && zq > M.s0_thr) {
       atomicOr(d.bond_bits + (kglob >> 5), 1u << (kglob & 31));
     } else {
       const float vol = volj * (rji > M.low_thr ? fmaf(-rji, M.inv_h, M.cu_h) : 1.f);
-      const float J = gauss ? M.j0 * ex2(r2 * M.j1) : fmaf(M.j1, rji, M.j0);
+      const float J = GAUSS ? M.j0 * ex2(r2 * M.j1) : fmaf(M.j1, rji, M.j0);
       th = fmaf(rji * cl, J * vol, th);
     }
   }
+}
+
+// the state-based law's record of a node: {theta (3K - 5G) / m_x, 15 G / m_x}
+__device__ __forceinline__ float2 state_record(double theta, double mx, const MixParticle &M) {
+  const double inv_m = 1.0 / mx;
+  return make_float2((float)(theta * M.tf_coef * inv_m), (float)(M.am_coef * inv_m));
+}
+
+__global__ void k_state_records(const __grid_constant__ DevData d) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= d.n_nodes || d.particles[d.ptid[i]].material != PDGPU_MAT_PDSTATE) return;
+  d.m_mixed[i] = state_record(d.theta[i], d.mx[i], d.mixp[d.ptid[i]]);
+}
+
+// 3-D: every node's displacement relative to its particle centre's, as the
+// tiles of the pre-pass and the bond loop stage it.  One pass over the nodes
+// (244 000 nodes: 4.3 us; pre-pass 65 -> 56 us, bond loop 74 -> 61) in place of a conversion per window node and tile, ~1 900 per
+// 128-node tile of R / h = 10 spheres, in both kernels.
+__global__ void __launch_bounds__(256) k_urel(const __grid_constant__ DevData d) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= d.n_nodes || d.ctrl->error) return;
+  const double2 *u = reinterpret_cast<const double2 *>(d.u);
+  const double2 a = u[2 * i], b = u[2 * i + 1];
+  const int64_t c = d.particles[d.ptid[i]].center;
+  const double2 ca = u[2 * c], cb = u[2 * c + 1];
+  d.urel[i] = make_float4((float)(a.x - ca.x), (float)(a.y - ca.y), (float)(b.x - cb.x), 0.f);
 }
 
 // the pre-pass over one staged tile: theta_i = 3 sum / m_x,i
@@ -269,9 +334,10 @@ __device__ __forceinline__ void tile_theta(const DevData &d, const BondTile &T, 
   const int col_off = (int)(kb - p.col0);
   const int bit_off = (int)(kb - 32 * p.word0);
   const int shift = sizeof(CT) == 2 ? (int)(M.start - T.win_begin) : (int)(-T.win_begin);
+  const View<DIM> N = V.from(shift);  // indexed by neighbour column
+  const CT *cols = s_col + col_off;
   const bool gauss = d.inf.type == PDGPU_INF_GAUSSIAN;
-  // a warp's 32 / LPN nodes go through the loop together; past the tile's end
-  // a group has an empty row
+  // as in tile_nodes: without tests first, again with them where they matter
   for (int64_t wb = T.node_begin + threadIdx.x / 32 * (32 / LPN); wb < T.node_end; wb += kThreadsFor<DIM, LPN> / LPN) {
     const int64_t pos = wb + (threadIdx.x & 31) / LPN;
     const bool in_tile = pos < T.node_end;
@@ -281,20 +347,36 @@ __device__ __forceinline__ void tile_theta(const DevData &d, const BondTile &T, 
     const int li = (int)(i - T.win_begin);
     float xi[3], ui[3], vi;
     V.node(li, xi, ui, vi);
-    float th = 0.f;
-    if (!any_broken<LPN>(s_bits, k0 + bit_off, k1 + bit_off)) {
+    float th = 0.f, zmax = 0.f;
+    bool test = any_broken<LPN>(s_bits, k0 + bit_off, k1 + bit_off);
+    if (!test) {
+      if (gauss) {
 #pragma unroll 2
-      for (int k = k0 + lane; k < k1; k += LPN)
-        pre_bond<DIM, true>(d, M, V, xi, ui, (int)s_col[k + col_off] + shift, false, gauss, kb + k, th);
-    } else {
+        for (int k = k0 + lane; k < k1; k += LPN)
+          pre_bond<DIM, false, true>(d, M, N, xi, ui, (int)cols[k], false, 0, th, zmax);
+      } else {
+#pragma unroll 4
+        for (int k = k0 + lane; k < k1; k += LPN)
+          pre_bond<DIM, false, false>(d, M, N, xi, ui, (int)cols[k], false, 0, th, zmax);
+      }
+    }
+    test |= gmax<LPN>(zmax) > M.s0_thr;
+    if (test) {
+      th = 0.f;
       for (int k = k0 + lane; k < k1; k += LPN) {
         const int b = k + bit_off;
         const bool broken = (s_bits[b >> 5] >> (b & 31)) & 1u;
-        pre_bond<DIM, false>(d, M, V, xi, ui, (int)s_col[k + col_off] + shift, broken, gauss, kb + k, th);
+        if (gauss) pre_bond<DIM, true, true>(d, M, N, xi, ui, (int)cols[k], broken, kb + k, th, zmax);
+        else pre_bond<DIM, true, false>(d, M, N, xi, ui, (int)cols[k], broken, kb + k, th, zmax);
       }
     }
+    __syncwarp();
     const double t = gsum<LPN>((double)th);
-    if (lane == 0 && in_tile) d.theta[i] = 3.0 * t / d.mx[i];
+    if (lane == 0 && in_tile) {
+      const double theta = 3.0 * t / d.mx[i];
+      d.theta[i] = theta;
+      d.m_mixed[i] = state_record(theta, d.mx[i], M);
+    }
   }
 }
 
@@ -538,7 +620,8 @@ __global__ void __launch_bounds__(kThreadsFor<DIM, LPN>) k_bonds_mixed(DevData d
       continue;
     }
     const int w = (int)(T.win_end - T.win_begin);
-    const Plan p = plan(DIM, state, (int)sizeof(CT), T.bond_begin, T.bond_end, T.node_begin, T.node_end, w);
+    const Plan p = plan(DIM, state, (int)sizeof(CT), T.bond_begin, T.bond_end, T.node_begin, T.node_end,
+                        T.win_begin, T.win_end);
     SymPlan q{};
     if constexpr (SYM) q = sym_plan(p, T.node_begin, T.node_end, T.slots);
     CT *s_col = reinterpret_cast<CT *>(smem);
@@ -547,13 +630,16 @@ __global__ void __launch_bounds__(kThreadsFor<DIM, LPN>) k_bonds_mixed(DevData d
     float4 *s_xv = reinterpret_cast<float4 *>(smem + p.off_xv);
     float2 *s_u2 = reinterpret_cast<float2 *>(smem + p.off_u);
     float4 *s_u4 = reinterpret_cast<float4 *>(smem + p.off_u);
-    float2 *s_m = reinterpret_cast<float2 *>(smem + p.off_m);
+    float2 *s_m = reinterpret_cast<float2 *>(smem + p.off_m) + (T.win_begin - p.m0);
 
     // columns, bitmap words, row offsets and constant node records of the
     // tile: bulk copies; then the claim of the next tile
     if (threadIdx.x == 0) {
       fence_async_smem();
-      bar_arrive_tx(&bar, p.col_bytes + p.bit_bytes + p.row_bytes + 16u * (uint32_t)w + (SYM ? q.meta_bytes : 0u));
+      bar_arrive_tx(&bar, p.col_bytes + p.bit_bytes + p.row_bytes + (DIM == 3 ? 32u : 16u) * (uint32_t)w + p.m_bytes +
+                              (SYM ? q.meta_bytes : 0u));
+      if constexpr (DIM == 3) bulk_load(s_u4, d.urel + T.win_begin, 16u * (uint32_t)w, &bar);
+      if (state) bulk_load(smem + p.off_m, d.m_mixed + p.m0, p.m_bytes, &bar);
       if constexpr (SYM) bulk_load(smem + q.off_meta, d.sym_meta + q.meta0, q.meta_bytes, &bar);
       if (p.col_bytes) bulk_load(s_col, col + p.col0, p.col_bytes, &bar);
       if (p.bit_bytes) bulk_load(s_bits, d.bond_bits + p.word0, p.bit_bytes, &bar);
@@ -563,26 +649,14 @@ __global__ void __launch_bounds__(kThreadsFor<DIM, LPN>) k_bonds_mixed(DevData d
     }
     const MixParticle M = d.mixp[T.particle];
 
-    // displacements of the window relative to the particle centre's
-    {
-      const int st = DIM == 2 ? 2 : 4;
-      double uc[DIM];
-#pragma unroll
-      for (int q = 0; q < DIM; q++) uc[q] = d.u[st * T.center + q];
+    // 2-D: displacements of the window relative to the particle centre's (in
+    // 3-D, where a tile's window is some fifteen times the tile, k_urel has
+    // written them once per node)
+    if constexpr (DIM == 2) {
+      const double2 uc = *reinterpret_cast<const double2 *>(d.u + 2 * T.center);
       for (int a = threadIdx.x; a < w; a += kThreadsFor<DIM, LPN>) {
-        const int64_t j = T.win_begin + a;
-        if constexpr (DIM == 2) {
-          const double2 uj = *reinterpret_cast<const double2 *>(d.u + 2 * j);
-          s_u2[a] = make_float2((float)(uj.x - uc[0]), (float)(uj.y - uc[1]));
-        } else {
-          const double2 u01 = *reinterpret_cast<const double2 *>(d.u + 4 * j);
-          const double u2 = d.u[4 * j + 2];
-          s_u4[a] = make_float4((float)(u01.x - uc[0]), (float)(u01.y - uc[1]), (float)(u2 - uc[2]), 0.f);
-        }
-        if (state) {
-          const double inv_m = 1.0 / d.mx[j];
-          s_m[a] = make_float2((float)(d.theta[j] * M.tf_coef * inv_m), (float)(M.am_coef * inv_m));
-        }
+        const double2 uj = *reinterpret_cast<const double2 *>(d.u + 2 * (T.win_begin + a));
+        s_u2[a] = make_float2((float)(uj.x - uc.x), (float)(uj.y - uc.y));
       }
     }
     __syncthreads();
@@ -741,6 +815,17 @@ void launch_pd_tiled_mixed(const DevData &d, const BondTile *t, const int *law_b
   }
 }
 
+// 3-D: the relative displacements the tiles stage, ahead of the pre-pass and
+// the bond loop
+void launch_urel(const DevData &d, cudaStream_t s) {
+  if (d.urel) mixed_loop::k_urel<<<(unsigned)((d.n_nodes + 255) / 256), 256, 0, s>>>(d);
+}
+// state records from the current dilatations and m_x (the pre-pass writes
+// them from then on)
+void launch_state_records(const DevData &d, cudaStream_t s) {
+  if (d.m_mixed) mixed_loop::k_state_records<<<(unsigned)((d.n_nodes + 255) / 256), 256, 0, s>>>(d);
+}
+
 // PD state pre-pass over the tiles of state-based particles, persistent like
 // the bond loop
 void launch_prepass_mixed(const DevData &d, const BondTile *t, const int *law_begin, int lanes, size_t smem,
@@ -760,7 +845,7 @@ void launch_prepass_mixed(const DevData &d, const BondTile *t, const int *law_be
 
 size_t tile_smem_mixed_main(int dim, bool state, bool col16, const BondTile &t, bool sym) {
   const mixed_loop::Plan p = mixed_loop::plan(dim, state, col16 ? 2 : 4, t.bond_begin, t.bond_end, t.node_begin,
-                                              t.node_end, t.win_end - t.win_begin);
+                                              t.node_end, t.win_begin, t.win_end);
   return sym ? mixed_loop::sym_plan(p, t.node_begin, t.node_end, t.slots).total : p.total;
 }
 

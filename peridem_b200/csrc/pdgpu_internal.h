@@ -273,6 +273,8 @@ struct DevData {
   int32_t *node_order;
   MixParticle *mixp;
   float4 *xv_mixed;  // per node {x, y, z, vol}: reference coordinates minus the centre's, FP32
+  float4 *urel;      // 3-D: displacement relative to the particle centre's, FP32, of this evaluation
+  float2 *m_mixed;   // state-based particles: {theta (3K - 5G) / m_x, 15 G / m_x}
   int32_t use16;
   float inf_p0, inf_p1;
 
@@ -412,6 +414,8 @@ void launch_prepass_tiled_fp64(const DevData &d, const BondTile *tiles, const in
                                size_t smem, cudaStream_t s);
 void launch_pd_tiled_mixed(const DevData &d, const BondTile *tiles, const int *law_begin, int lanes,
                            size_t smem, cudaStream_t s);
+void launch_urel(const DevData &d, cudaStream_t s);
+void launch_state_records(const DevData &d, cudaStream_t s);
 // persistent PD state pre-pass of the mixed form over the state-based tiles
 void launch_prepass_mixed(const DevData &d, const BondTile *tiles, const int *law_begin, int lanes,
                           size_t smem, cudaStream_t s);

@@ -512,10 +512,11 @@ int alloc_col16(pdgpu_ctx *ctx) {
   return PDGPU_OK;
 }
 
-// node constants of the FP64 form that follow from m_x (set again when a
-// later call changes m_x)
-int fp64_node_constants(pdgpu_ctx *ctx) {
-  launch_fp64_setup(ctx->d, ctx->stream);
+// node constants that follow from m_x (and, in the mixed form, the dilatations):
+// set again when a later call changes those
+int node_constants(pdgpu_ctx *ctx) {
+  if (ctx->d.precision == PDGPU_PREC_FP64) launch_fp64_setup(ctx->d, ctx->stream);
+  else launch_state_records(ctx->d, ctx->stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
   return PDGPU_OK;
@@ -539,7 +540,7 @@ int prepare_fp64(pdgpu_ctx *ctx) {
   dfree(ctx, out);
   // the kernels that read the bond data from global memory check every root
   ctx->stage_level0 = outside ? kStageLevels - 1 : 0;
-  return fp64_node_constants(ctx);
+  return node_constants(ctx);
 }
 
 // FP32 constants per particle for the mixed-precision bond loop
@@ -614,12 +615,13 @@ int prepare_mixed(pdgpu_ctx *ctx) {
   CK(cudaMemcpy(d.mixp, mp.data(), mp.size() * sizeof(MixParticle), cudaMemcpyHostToDevice));
   TRY(alloc_col16(ctx));
   TRY(dalloc(ctx, &d.xv_mixed, N));
+  if (d.dim == 3) TRY(dalloc(ctx, &d.urel, N));
+  for (const auto &P : ctx->hp)
+    if (P.material == PDGPU_MAT_PDSTATE && P.compute_force && !d.m_mixed) TRY(dalloc(ctx, &d.m_mixed, N + 2));
   d.inf_p0 = (float)d.inf.p0;
   d.inf_p1 = (float)d.inf.p1;
   launch_mixed_setup(d, ctx->stream);
-  CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(ctx->stream));
-  return PDGPU_OK;
+  return node_constants(ctx);
 }
 
 // The learned surrogate's list of bond-loop tiles (written each step by the
@@ -676,7 +678,7 @@ void choose_tiling(pdgpu_ctx *ctx) {
   const bool choose = ctx->pd_lanes <= 0 && ctx->tile_nodes <= 0;
   if (ctx->pd_lanes <= 0) ctx->pd_lanes = lanes0;
   if (choose) {
-    const int threads = d.dim == 3 ? 512 : 256;
+    const int threads = d.dim == 3 ? 512 : (mixed ? 128 : 256);
     const int64_t room = (int64_t)sm_count() * (d.dim == 2 ? 3 : 1);  // FP64 CTAs at once
     int64_t active = 0;
     for (const auto &P : ctx->hp) active += P.compute_force ? P.end - P.start : 0;
@@ -1053,6 +1055,7 @@ void pd_forces(pdgpu_ctx *ctx) {
   DevData &d = ctx->d;
   cudaStream_t s = ctx->stream;
   const bool mixed = d.precision == PDGPU_PREC_MIXED;
+  if (d.urel) run(ctx, "relative_u", [&] { launch_urel(d, s); });
   if (ctx->state_prepass) {
     if (mixed)
       run(ctx, "pd_prepass_mixed", [&] {
@@ -1206,6 +1209,7 @@ cudaError_t graph_step(pdgpu_ctx *ctx, const char **where) {
     if (e != cudaSuccess) return e;
   }
   // main: bond loop
+  launch_urel(d, s);
   if (ctx->state_prepass) {
     if (mixed) launch_prepass_mixed(d, ctx->tiles, ctx->tile_law, ctx->pd_lanes, ctx->tile_smem_pd, s);
     else launch_prepass_tiled_fp64(d, ctx->tiles, ctx->tile_law, ctx->pd_lanes, ctx->tile_stage, ctx->tile_smem_pd, s);
@@ -1579,7 +1583,7 @@ int pdgpu_upload_mx(pdgpu_ctx *ctx, const double *mx) {
   if (!ctx->nodes) return fail(ctx, PDGPU_ERR_STATE, "upload nodes first");
   CK(cudaMemcpy(ctx->d.mx, mx, ctx->d.n_nodes * 8, cudaMemcpyHostToDevice));
   ctx->mx = true;
-  return ctx->prepared && ctx->d.precision == PDGPU_PREC_FP64 ? fp64_node_constants(ctx) : PDGPU_OK;
+  return ctx->prepared ? node_constants(ctx) : PDGPU_OK;
 }
 
 int pdgpu_compute_mx(pdgpu_ctx *ctx) {
@@ -1591,7 +1595,7 @@ int pdgpu_compute_mx(pdgpu_ctx *ctx) {
   CK(cudaGetLastError());
   TRY(device_error(ctx));
   ctx->mx = true;
-  return ctx->prepared && ctx->d.precision == PDGPU_PREC_FP64 ? fp64_node_constants(ctx) : PDGPU_OK;
+  return ctx->prepared ? node_constants(ctx) : PDGPU_OK;
 }
 
 int pdgpu_add_displacement_bc(pdgpu_ctx *ctx, const pdgpu_bc_set *set, const uint8_t *psel,
@@ -2938,6 +2942,7 @@ int pdgpu_load_state(pdgpu_ctx *ctx, const char *path) {
   TRY(ul(ctx, d.Z, Z));
   TRY(ul(ctx, d.vmag, vmag));
   TRY(ul(ctx, d.theta, theta));
+  TRY(node_constants(ctx));
   TRY(ul(ctx, d.bond_bits, bits));
   CK(cudaMemcpyAsync(d.ctrl, &c, sizeof c, cudaMemcpyHostToDevice, ctx->stream));
   if (multi) {
