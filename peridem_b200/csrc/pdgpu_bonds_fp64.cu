@@ -39,6 +39,7 @@
 
 #include "pdgpu_bulk.cuh"
 #include "pdgpu_internal.h"
+#include "pdgpu_pdl.cuh"
 
 namespace pdgpu {
 namespace {
@@ -305,6 +306,8 @@ __global__ void __launch_bounds__(kThreads64<DIM>, DIM == 2 ? 3 : 1)
   constexpr int kT = kThreads64<DIM>;
   constexpr bool kState = LAW == LAW_STATE && !PRE;
   constexpr bool kStaged = !std::is_void<COL>::value;
+  pdl_start();
+  pdl_wait();
   if (d.ctrl->error) return;
   const BondTile T = tiles[blockIdx.x];
   const DevParticle &P = d.particles[T.particle];
@@ -486,7 +489,9 @@ __global__ void k_fp64_range(const __grid_constant__ DevData d, int32_t *outside
 
 template <int DIM, int LPN, int LAW, bool PRE, typename COL>
 void launch_one(const DevData &d, const BondTile *t, int n, int stage, size_t smem, cudaStream_t s) {
-  k_bonds_fp64<DIM, LPN, LAW, PRE, COL><<<n, kThreads64<DIM>, smem, s>>>(d, t, stage);
+  // behind the pre-pass (see launch_one of the FP32 form for the others)
+  if constexpr (LAW == LAW_STATE && !PRE) launch_dependent(k_bonds_fp64<DIM, LPN, LAW, PRE, COL>, n, kThreads64<DIM>, smem, s, d, t, stage);
+  else k_bonds_fp64<DIM, LPN, LAW, PRE, COL><<<n, kThreads64<DIM>, smem, s>>>(d, t, stage);
 }
 
 template <int DIM, int LAW, bool PRE>

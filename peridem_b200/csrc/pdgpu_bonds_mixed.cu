@@ -32,6 +32,7 @@
 
 #include "pdgpu_bulk.cuh"
 #include "pdgpu_internal.h"
+#include "pdgpu_pdl.cuh"
 
 namespace pdgpu {
 
@@ -315,6 +316,7 @@ __global__ void k_state_records(const __grid_constant__ DevData d) {
 // (244 000 nodes: 4.3 us; pre-pass 65 -> 56 us, bond loop 74 -> 61) in place of a conversion per window node and tile, ~1 900 per
 // 128-node tile of R / h = 10 spheres, in both kernels.
 __global__ void __launch_bounds__(256) k_urel(const __grid_constant__ DevData d) {
+  pdl_start();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= d.n_nodes || d.ctrl->error) return;
   const double2 *u = reinterpret_cast<const double2 *>(d.u);
@@ -590,6 +592,8 @@ __global__ void __launch_bounds__(kThreadsFor<DIM, LPN>) k_bonds_mixed(DevData d
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar;
   __shared__ int s_tile[2];
+  pdl_start();
+  pdl_wait();
   if (d.ctrl->error) return;
   constexpr bool state = LAW == LAW_STATE && !PRE;  // the pre-pass needs no m, theta stage
   // learned surrogate: off check steps, its particles' tiles are left out —
@@ -714,7 +718,12 @@ template <int DIM, int LPN, int LAW, typename CT, bool PRE = false, bool SYM = f
 void launch_one(const DevData &d, const CT *col, const BondTile *t, int n, size_t smem, cudaStream_t s) {
   auto *k = k_bonds_mixed<DIM, LPN, LAW, CT, PRE, SYM>;
   constexpr int kT = kThreadsFor<DIM, LPN>;
-  k<<<bond_grid(k, kT, smem, n), kT, smem, s>>>(d, t, n, col);
+  const int g = bond_grid(k, kT, smem, n);
+  // in 3-D k_urel, the pre-pass or another law's launch is ahead; in 2-D the
+  // contact rebuild may be, and CTAs that came before the contact pass's
+  // would leave those no room
+  if constexpr (DIM == 3) launch_dependent(k, g, kT, smem, s, d, t, n, col);
+  else k<<<g, kT, smem, s>>>(d, t, n, col);
 }
 
 template <int DIM, int LAW, typename CT, bool PRE = false, bool SYM = false>

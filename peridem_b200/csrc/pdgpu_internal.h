@@ -213,6 +213,7 @@ struct DevData {
   int64_t cell_cap;  // max nodes in one cell handled by the in-cell sort
 
   // particle-wall damping pairs
+  int32_t has_walls;  // some particle is a wall
   int32_t wp_cap;
   int32_t *wp, *wp_cnt;
   double *fdamp;  // n_particles * 4

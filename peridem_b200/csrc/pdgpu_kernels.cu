@@ -15,6 +15,7 @@
 #include <cstdint>
 
 #include "pdgpu_internal.h"
+#include "pdgpu_pdl.cuh"
 
 namespace pdgpu {
 
@@ -439,28 +440,36 @@ __global__ void __launch_bounds__(kBlock) k_step_begin(const __grid_constant__ D
   __shared__ int last;
   __shared__ __align__(8) CtrlState s_ctrl;
   static_assert(sizeof(CtrlState) % 8 == 0 && sizeof(CtrlState) / 8 <= kBlock, "CtrlState copy");
+  pdl_start();
+  // CTAs run in reverse node order: the boundary-condition nodes (walls, at
+  // the end of the node array) then start in the first wave.  Each thread
+  // takes kBeginNodes nodes, kBlock apart, and issues every load of all of
+  // them before the first update; what no kernel writes, ahead of the wait.
+  const int64_t base = (int64_t)(gridDim.x - 1 - blockIdx.x) * (kBlock * kBeginNodes) + threadIdx.x;
+  uint8_t fl[kBeginNodes], fix[kBeginNodes];
+  int32_t pid[kBeginNodes];
+#pragma unroll
+  for (int k = 0; k < kBeginNodes; k++) {
+    const int64_t i = base + (int64_t)k * kBlock;
+    fl[k] = 0;
+    if (i < d.n_nodes) {
+      fl[k] = d.flags[i];
+      fix[k] = d.fix[i];
+      pid[k] = d.ptid[i];
+    }
+  }
+  pdl_wait();
   // every block copies the step-control state now, while its nodes load: the
   // last block's step control then starts without a chain of cold loads
   if (threadIdx.x < sizeof(CtrlState) / 8)
     reinterpret_cast<uint64_t *>(&s_ctrl)[threadIdx.x] = reinterpret_cast<const uint64_t *>(d.ctrl)[threadIdx.x];
-  // CTAs run in reverse node order: the boundary-condition nodes (walls, at
-  // the end of the node array) then start in the first wave.  Each thread
-  // takes kBeginNodes nodes, kBlock apart, and issues every load of all of
-  // them before the first update.
-  const int64_t base = (int64_t)(gridDim.x - 1 - blockIdx.x) * (kBlock * kBeginNodes) + threadIdx.x;
   double vm = 0.0;
   if (!d.ctrl->error) {
-    uint8_t fl[kBeginNodes], fix[kBeginNodes];
-    int32_t pid[kBeginNodes];
     double v[kBeginNodes][3], u[kBeginNodes][3], x[kBeginNodes][3], f[kBeginNodes][3];
 #pragma unroll
     for (int k = 0; k < kBeginNodes; k++) {
       const int64_t i = base + (int64_t)k * kBlock;
-      fl[k] = 0;
       if (i < d.n_nodes) {
-        fl[k] = d.flags[i];
-        fix[k] = d.fix[i];
-        pid[k] = d.ptid[i];
         ldv<DIM>(d.v, i, v[k]);
         ldv<DIM>(d.u, i, u[k]);
         ldv<DIM>(d.x, i, x[k]);
@@ -972,6 +981,7 @@ __global__ void __launch_bounds__(kCoopBlock) k_contact_rebuild(DevData d, uint8
                                                                int64_t *bsum) {
   extern __shared__ __align__(16) unsigned char cand_smem[];
   CandWarp<DIM> *stage = reinterpret_cast<CandWarp<DIM> *>(cand_smem);
+  pdl_wait();
   if (d.ctrl->error) return;
   if (!d.ctrl->update) {
     list_live_tiles(d);
@@ -1367,6 +1377,7 @@ template <int DIM>
 __global__ void __launch_bounds__(kBlock) k_contact_warp(const __grid_constant__ DevData d) {
   __shared__ ContactPair cps[kZonePairsSmem];
   __shared__ double scr[kBlock];
+  pdl_start();
   const int l32 = threadIdx.x & 31;
   const int nz = d.n_zones;
   const bool tab = nz * nz <= kZonePairsSmem;
@@ -1606,6 +1617,7 @@ __global__ void __launch_bounds__(kDampBlock) k_damp_walls(const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int p = blockIdx.x * (kDampBlock / 32) + warp;
   const int cap = min(d.wp_cap, kWallSort);  // the capacity is validated on the host
+  pdl_wait();
   const int nw = p < d.n_particles && !d.ctrl->error ? min(d.wp_cnt[p], cap) : 0;
   if (nw > 0 && nw <= kWallWarp) {  // ordered by counting
     int32_t *mine = wn + warp * (2 * kWallWarp);
@@ -1895,6 +1907,7 @@ constexpr int kEndNodes = 2;  // nodes per thread of the step-end kernel
 template <int DIM, bool VERLET>
 __global__ void __launch_bounds__(kBlock) k_step_end(const __grid_constant__ DevData d, int post) {
   __shared__ int last;
+  pdl_start();
   const int64_t n_step = d.ctrl->n;
   // each thread takes kEndNodes nodes, kBlock apart, and issues the node
   // loads of all of them (independent of their flags) before the sums
@@ -2147,8 +2160,19 @@ static cudaError_t rebuild_dim(const DevData &d, uint8_t bit, int64_t *bsum, int
                                cudaStream_t s) {
   DevData dd = d;
   void *args[] = {(void *)&dd, (void *)&bit, (void *)&bsum};
-  return cudaLaunchCooperativeKernel((const void *)k_contact_rebuild<DIM, LPN>, dim3(grid),
-                                     dim3(kCoopBlock), args, cand_stage_bytes<DIM>(), s);
+  cudaLaunchAttribute at[2]{};
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(kCoopBlock);
+  c.dynamicSmemBytes = cand_stage_bytes<DIM>();
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 2;
+  return cudaLaunchKernelExC(&c, (const void *)k_contact_rebuild<DIM, LPN>, args);
 }
 
 int rebuild_grid_blocks(const DevData &d, int lanes) {
@@ -2220,8 +2244,9 @@ void launch_scene_post(const DevData &d, cudaStream_t s) {
 }
 
 void launch_damping(const DevData &d, cudaStream_t s) {
-  if (d.n_particles <= 0) return;
-  PDGPU_DIM_DISPATCH(d, k_damp_walls, <<<blocks_for(d.n_particles, kDampBlock / 32), kDampBlock, 0, s>>>(d));
+  if (!d.has_walls) return;
+  launch_dependent(d.dim == 2 ? k_damp_walls<2> : k_damp_walls<3>, blocks_for(d.n_particles, kDampBlock / 32),
+                   kDampBlock, 0, s, d);
 }
 
 void launch_external(const DevData &d, cudaStream_t s) {
@@ -2232,13 +2257,8 @@ void launch_external(const DevData &d, cudaStream_t s) {
 
 void launch_step_begin(const DevData &d, int verlet, cudaStream_t s) {
   const unsigned g = blocks_for(d.n_nodes, kBlock * kBeginNodes);
-  if (d.dim == 2) {
-    if (verlet) k_step_begin<2, true><<<g, kBlock, 0, s>>>(d);
-    else k_step_begin<2, false><<<g, kBlock, 0, s>>>(d);
-  } else {
-    if (verlet) k_step_begin<3, true><<<g, kBlock, 0, s>>>(d);
-    else k_step_begin<3, false><<<g, kBlock, 0, s>>>(d);
-  }
+  if (d.dim == 2) launch_dependent(verlet ? k_step_begin<2, true> : k_step_begin<2, false>, g, kBlock, 0, s, d);
+  else launch_dependent(verlet ? k_step_begin<3, true> : k_step_begin<3, false>, g, kBlock, 0, s, d);
 }
 
 void launch_step_end(const DevData &d, int verlet, int post, cudaStream_t s) {

@@ -1468,6 +1468,8 @@ int pdgpu_upload_particles(pdgpu_ctx *ctx, int64_t np, const pdgpu_particle *p) 
   }
   DevData &d = ctx->d;
   d.n_particles = (int32_t)np;
+  d.has_walls = 0;
+  for (const auto &P : ctx->hp) d.has_walls |= P.type == 1;
   TRY(dalloc(ctx, &d.particles, np));
   CK(cudaMemcpy(d.particles, ctx->hp.data(), np * sizeof(DevParticle), cudaMemcpyHostToDevice));
   ctx->particles = true;
