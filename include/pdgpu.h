@@ -478,7 +478,8 @@ PDGPU_API int pdgpu_write_strain_vtu(pdgpu_ctx *ctx, const char *path, int64_t n
  * passes each grid-wide barrier, in order: start, cells cleared, nodes
  * counted per cell, cell offsets scanned, nodes scattered, cells sorted,
  * candidates counted, row offsets scanned, compaction offsets scanned,
- * lists compacted, and the first CTA's share of the fill done (11 marks).
+ * lists compacted, and the first CTA's share of the fill done (11 marks;
+ * steps that one pass does together have the same mark).
  * pdgpu_rebuild_phases copies the marks of the latest rebuild (up to cap)
  * and sets *count. */
 PDGPU_API int pdgpu_enable_rebuild_phases(pdgpu_ctx *ctx, int32_t on);

@@ -204,11 +204,13 @@ struct DevData {
   unsigned long long *phase_ns;  // rebuild phase clock (null: off), kRebuildPhases marks
   uint8_t *c_hit;  // per candidate entry, this step: inside the largest contact radius
   int64_t *c_cnt;  // per-node candidate counts of the last rebuild
-  int64_t *c_tmp;  // N+1 scratch for the compaction scan
   int32_t *c_nodes;  // nodes with candidates, ascending
   int32_t contact_grid;  // blocks of the contact node pass
   Grid grid;
   int32_t *cell_of, *cell_cnt, *cell_start, *cell_fill, *cell_tmp, *cell_nodes;
+  // contact rebuild, per node in cell order: its particle and position
+  int32_t *cell_p;
+  double *cell_x;
   int32_t *cell_pid;  // contact rebuild: the particle of a cell's nodes when they share one, else -1
   int64_t cell_cap;  // max nodes in one cell handled by the in-cell sort
 
@@ -439,9 +441,8 @@ cudaError_t launch_strain_tet(const DevData &d, int64_t n_elem, const int64_t *c
                               const double *lam, const double *mu, double *xq, double *strain, double *stress,
                               cudaStream_t s);
 constexpr int kRebuildPhases = 16;
-int rebuild_grid_blocks(const DevData &d, int lanes);
-cudaError_t launch_contact_rebuild(const DevData &d, int64_t *bsum, int grid, int lanes, int init,
-                                   cudaStream_t s);
+int rebuild_grid_blocks(const DevData &d);
+cudaError_t launch_contact_rebuild(const DevData &d, int64_t *bsum, int grid, int init, cudaStream_t s);
 void launch_damping(const DevData &d, cudaStream_t s);
 void launch_scene_post(const DevData &d, cudaStream_t s);  // per-scene test output of an ensemble
 void launch_external(const DevData &d, cudaStream_t s);

@@ -11,6 +11,7 @@
 #include <cooperative_groups.h>
 #include <cub/cub.cuh>
 
+#include <algorithm>
 #include <cfloat>
 #include <cstdint>
 
@@ -636,7 +637,7 @@ __device__ bool grid_bar(CtrlState *c) {
           atomicCAS(&c->error, 0, DEV_ERR_BARRIER_TIMEOUT);
           break;
         }
-        __nanosleep(128);
+        __nanosleep(32);
       }
     }
     __threadfence();
@@ -711,176 +712,150 @@ __device__ bool grid_scan(CtrlState *gc, F in, Tout *out, int64_t n, int64_t *bs
 }
 
 
-// Candidate pass, cell-centric: a warp takes a centre cell and stages its
-// neighbourhood (the 3^DIM cells around it, z, y, x ascending; each cell's
-// nodes ascending) in its own slice of shared memory, in chunks; every
-// searching node of the centre cell scans the staged list in that order with
-// the strict test sum_d (q_d - p_d)^2 < r^2 (nanoflann's L2 order), skipping
-// nodes of its own particle.  Each node's candidates thus come in (cell, node
-// index) order.  COUNT writes c_cnt for every node; FILL writes the columns.
-// Per-warp staging of the candidate pass, in dynamic shared memory: a chunk
-// of neighbourhood entries (position, node, particle) and the state of up to
-// kCandCentres centre nodes (position, particle, running count / output slot).
-constexpr int kCandChunk = 256;
-constexpr int kCandCentres = 64;
-
-template <int DIM>
-struct CandWarp {
-  double x[DIM][kCandChunk];
-  double q[DIM][kCandCentres];
-  int64_t out[kCandCentres];
-  int32_t j[kCandChunk], p[kCandChunk];
-  int32_t ci[kCandCentres], pi[kCandCentres];
-  int32_t nb_s[DIM == 3 ? 27 : 9], nb_off[(DIM == 3 ? 27 : 9) + 1];
-};
-
-template <int DIM>
-constexpr size_t cand_stage_bytes() {
-  return sizeof(CandWarp<DIM>) * (kCoopBlock / 32);
+// Exclusive scans of the candidate counts and of the nodes that have any, in
+// one pass over the nodes: emit(i, count, row start, compacted position); the
+// last block's totals go to tot[0], tot[1].  bsum: 2 values per block.
+template <class Emit>
+__device__ bool scan_rows(CtrlState *gc, const int64_t *cnt, int64_t n, int64_t *bsum, int64_t (&tot)[2], Emit emit) {
+  __shared__ int64_t wsum[2][kCoopBlock / 32];
+  __shared__ int64_t carry[2];
+  const int64_t nb = gridDim.x;
+  const int64_t chunk = (n + nb - 1) / nb;
+  const int64_t b0 = min(n, blockIdx.x * chunk), b1 = min(n, b0 + chunk);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // sum of two values over the block, in t[0], t[1] of thread 0
+  auto block_sum = [&](int64_t (&t)[2]) {
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      for (int o = 16; o > 0; o >>= 1) t[q] += __shfl_xor_sync(0xffffffffu, t[q], o);
+      if (lane == 0) wsum[q][warp] = t[q];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int q = 0; q < 2; q++) {
+        t[q] = 0;
+        for (int w = 0; w < kCoopBlock / 32; w++) t[q] += wsum[q][w];
+      }
+  };
+  int64_t t[2] = {0, 0};
+  for (int64_t k = b0 + threadIdx.x; k < b1; k += blockDim.x) {
+    const int64_t c = cnt[k];
+    t[0] += c;
+    t[1] += c > 0;
+  }
+  block_sum(t);
+  if (threadIdx.x == 0) {
+    bsum[2 * blockIdx.x] = t[0];
+    bsum[2 * blockIdx.x + 1] = t[1];
+  }
+  if (!grid_bar(gc)) return false;
+  // carry = sum of the earlier blocks' totals (integers: any order gives the
+  // same sum), read past L1, which may hold this array from an earlier scan
+  t[0] = t[1] = 0;
+  for (int64_t k = threadIdx.x; k < blockIdx.x; k += blockDim.x) {
+    t[0] += __ldcg(bsum + 2 * k);
+    t[1] += __ldcg(bsum + 2 * k + 1);
+  }
+  block_sum(t);
+  if (threadIdx.x == 0) carry[0] = t[0], carry[1] = t[1];
+  __syncthreads();
+  for (int64_t base = b0; base < b1; base += blockDim.x) {
+    const int64_t k = base + threadIdx.x;
+    const int64_t v[2] = {k < b1 ? cnt[k] : 0, k < b1 && cnt[k] > 0 ? 1 : 0};
+    int64_t incl[2] = {v[0], v[1]};
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, incl[q], o);
+        if (lane >= o) incl[q] += y;
+      }
+      if (lane == 31) wsum[q][warp] = incl[q];
+    }
+    __syncthreads();
+    int64_t off[2] = {carry[0], carry[1]};
+    for (int w = 0; w < warp; w++) off[0] += wsum[0][w], off[1] += wsum[1][w];
+    if (k < b1) emit(k, v[0], off[0] + incl[0] - v[0], off[1] + incl[1] - v[1]);
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int w = 0; w < kCoopBlock / 32; w++) carry[0] += wsum[0][w], carry[1] += wsum[1][w];
+    __syncthreads();
+  }
+  tot[0] = carry[0];
+  tot[1] = carry[1];
+  return true;
 }
 
-template <int DIM, int LPN, bool FILL>
-__device__ void cand_cells(const DevData &d, uint8_t search_bit, CandWarp<DIM> *stage) {
-  constexpr int kWarps = kCoopBlock / 32;
-  constexpr int kNb = DIM == 3 ? 27 : 9;
-  const int wl = threadIdx.x >> 5, l32 = threadIdx.x & 31;
-  CandWarp<DIM> &W = stage[wl];
+// Candidate search: the nodes of the 3^DIM cells around a node's own (z, y, x
+// ascending; each cell's nodes ascending), those of its own particle skipped,
+// with the strict test sum_d (q_d - p_d)^2 < r^2 (nanoflann's L2 order).  A cell
+// whose nodes all belong to the searching node's particle is skipped whole
+// (cell_pid).  Particle and position of the nodes are read in cell order
+// (cell_p, cell_x), so an entry costs one round of loads.
+//
+// Count pass: LPN lanes per node, nodes in cell order, so that the groups of a
+// warp walk the same few cells and read the same entries.  Bound by the latency
+// of its loads at 1 024 threads per SM.  Against a warp per cell with the
+// neighbourhood staged in shared memory (B200, us): 2-D, 332 000 nodes 82 -> 30
+// (1 / 4 / 8 lanes per node: 40 / 37 / 58), 1.3 M nodes 176 -> 92; 3-D, 244 000
+// nodes 82 -> 50 (8 lanes 85, 16 lanes 142), 95 000 nodes 78 -> 30.
+constexpr int kCandLanes2 = 2, kCandLanes3 = 4;
+
+template <int DIM, int LPN>
+__device__ void cand_count(const DevData &d, uint8_t search_bit) {
+  constexpr int kUnroll = 4;
   const Grid G = d.grid;
   const double r = d.ctrl->radius;
   const double r2 = r * r;
-  const int lane = threadIdx.x % LPN;
-  const unsigned gm = group_mask<LPN>();
-  const unsigned lane_base = (threadIdx.x & 31u) / LPN * LPN;
-  constexpr int kGroups = 32 / LPN;
-  const int grp = l32 / LPN;
-  const int64_t nwarps = (int64_t)gridDim.x * kWarps;
-  for (int64_t c = (int64_t)blockIdx.x * kWarps + wl; c < G.ncells; c += nwarps) {
-    const int s_c = d.cell_start[c], e_c = d.cell_start[c + 1];
-    if (s_c == e_c) continue;  // warp-uniform
-    {
-      // lane t takes neighbour cell t in traversal order (z, y, x
-      // ascending); cells outside the grid contribute no nodes
-      const int t = l32;
-      const int cx0 = (int)(c % G.dims[0]);
-      const int cy0 = (int)((c / G.dims[0]) % G.dims[1]);
-      const int cz0 = DIM == 3 ? (int)(c / ((int64_t)G.dims[0] * G.dims[1])) : 0;
-      int a = 0, cnt = 0;
-      const int32_t pc_cell = d.cell_pid[c];
-      if (t < kNb) {
-        const int cx = cx0 + t % 3 - 1, cy = cy0 + (t / 3) % 3 - 1, cz = DIM == 3 ? cz0 + t / 9 - 1 : 0;
-        if (cx >= 0 && cx < G.dims[0] && cy >= 0 && cy < G.dims[1] && cz >= 0 &&
-            cz < (DIM == 3 ? G.dims[2] : 1)) {
-          const int cell = cx + G.dims[0] * (cy + G.dims[1] * cz);
-          // a centre cell of one particle finds nothing in a neighbour cell
-          // of that same particle
-          if (pc_cell < 0 || d.cell_pid[cell] != pc_cell) {
-            a = d.cell_start[cell];
-            cnt = d.cell_start[cell + 1] - a;
-          }
-        }
-      }
-      int incl = cnt;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (t >= o) incl += y;
-      }
-      if (t < kNb) {
-        W.nb_s[t] = a;
-        W.nb_off[t] = incl - cnt;
-      }
-      if (t == kNb - 1) W.nb_off[kNb] = incl;
-    }
-    __syncwarp();
-    const int total = W.nb_off[kNb];
-    if (total == 0) {
-      // every neighbour cell culled: no candidate for any node of this cell
-      for (int a = s_c + l32; a < e_c; a += 32) d.c_cnt[d.cell_nodes[a]] = 0;
-      __syncwarp();  // the warp's stage is reused by the next cell
-      continue;
-    }
-    // centre nodes in sets of up to kCandCentres (one set unless the cell is crowded)
-    for (int sb = s_c; sb < e_c; sb += kCandCentres) {
-      const int nc = min(kCandCentres, e_c - sb);
-      // particle of the centre cell's first node: a chunk whose entries and
-      // searching centres all belong to it cannot produce a candidate
-      const int32_t pc = d.ptid[d.cell_nodes[sb]];
-      bool mixed_centres = false;
-      for (int a = l32; a < nc; a += 32) {
-        const int32_t i = d.cell_nodes[sb + a];
-        const bool search = (d.flags[i] & search_bit) != 0;
+  const int sub = threadIdx.x % LPN;
+  const int64_t groups = (int64_t)gridDim.x * blockDim.x / LPN;
+  // all lanes of a warp stay in the loop together
+  for (int64_t a0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x - (threadIdx.x & 31)) / LPN; a0 < d.n_nodes;
+       a0 += groups) {
+    const int64_t a = a0 + (threadIdx.x & 31) / LPN;
+    int64_t n = 0;
+    int32_t i = -1;
+    if (a < d.n_nodes) {
+      i = d.cell_nodes[a];
+      const int cell0 = d.cell_of[i];
+      if (d.flags[i] & search_bit) {
         double q[3];
-        ldv<DIM>(d.x, i, q);
+        ldv<DIM>(d.cell_x, a, q);
+        const int32_t pi = d.cell_p[a];
+        const int cx0 = cell0 % G.dims[0], cy0 = cell0 / G.dims[0] % G.dims[1];
+        const int cz0 = DIM == 3 ? cell0 / G.dims[0] / G.dims[1] : 0;
+        const int zlo = DIM == 3 ? max(cz0 - 1, 0) : 0, zhi = DIM == 3 ? min(cz0 + 1, G.dims[2] - 1) : 0;
+        for (int cz = zlo; cz <= zhi; cz++)
+          for (int cy = max(cy0 - 1, 0); cy <= min(cy0 + 1, G.dims[1] - 1); cy++)
+            for (int cx = max(cx0 - 1, 0); cx <= min(cx0 + 1, G.dims[0] - 1); cx++) {
+              const int cell = cx + G.dims[0] * (cy + G.dims[1] * cz);
+              if (d.cell_pid[cell] == pi) continue;
+              const int e = d.cell_start[cell + 1];
+              for (int b = d.cell_start[cell] + sub; b < e; b += LPN * kUnroll) {
+                int32_t pb[kUnroll];
+                double pos[kUnroll][3];
 #pragma unroll
-        for (int t = 0; t < DIM; t++) W.q[t][a] = q[t];
-        W.ci[a] = i;
-        W.pi[a] = search ? d.ptid[i] : -2;  // -2: not searching
-        W.out[a] = FILL && search ? d.c_row[i] : 0;
-        if (search && W.pi[a] != pc) mixed_centres = true;
-      }
-      mixed_centres = __any_sync(0xffffffffu, mixed_centres);
-      for (int base = 0; base < total; base += kCandChunk) {
-        const int n = min(kCandChunk, total - base);
-        __syncwarp();  // the previous chunk is no longer read
-        for (int a = l32; a < n; a += 32) {
-          const int g = base + a;
-          int k = 0;
-          while (k + 1 < kNb && W.nb_off[k + 1] <= g) k++;
-          const int32_t j = d.cell_nodes[W.nb_s[k] + (g - W.nb_off[k])];
-          double p[3];
-          ldv<DIM>(d.x, j, p);
-#pragma unroll
-          for (int t = 0; t < DIM; t++) W.x[t][a] = p[t];
-          W.j[a] = j;
-          W.p[a] = d.ptid[j];
-        }
-        __syncwarp();
-        bool other = mixed_centres;
-        for (int a = l32; a < n && !other; a += 32) other = W.p[a] != pc;
-        if (!__any_sync(0xffffffffu, other)) continue;  // one particle only: no candidates here
-        for (int cb = 0; cb < nc; cb += kGroups) {
-          const int cc = cb + grp;
-          const int32_t pi = cc < nc ? W.pi[cc] : -2;
-          const bool search = pi != -2;
-          double q[3] = {0.0, 0.0, 0.0};
-          int64_t out = 0, out_end = 0;
-          if (search) {
-#pragma unroll
-            for (int t = 0; t < DIM; t++) q[t] = W.q[t][cc];
-            out = W.out[cc];
-            if (FILL) out_end = d.c_row[W.ci[cc] + 1];
-          }
-          for (int b0 = 0; b0 < n; b0 += LPN) {
-            const int a = b0 + lane;
-            bool hit = false;
-            int32_t j = -1;
-            if (search && a < n) {
-              j = W.j[a];
-              if (W.p[a] != pi) {
-                double dd = 0.0;
-#pragma unroll
-                for (int t = 0; t < DIM; t++) {
-                  const double df = q[t] - W.x[t][a];
-                  dd += df * df;
+                for (int k = 0; k < kUnroll; k++) {
+                  const int c = min(b + k * LPN, e - 1);
+                  pb[k] = b + k * LPN < e ? d.cell_p[c] : pi;
+                  ldv<DIM>(d.cell_x, c, pos[k]);
                 }
-                hit = dd < r2;
+#pragma unroll
+                for (int k = 0; k < kUnroll; k++) {
+                  double dd = 0.0;
+#pragma unroll
+                  for (int t = 0; t < DIM; t++) {
+                    const double df = q[t] - pos[k][t];
+                    dd += df * df;
+                  }
+                  n += pb[k] != pi && dd < r2;
+                }
               }
             }
-            const unsigned bal = (__ballot_sync(gm, hit) & gm) >> lane_base;
-            if (FILL && hit) {
-              const int64_t at = out + __popc(bal & ((1u << lane) - 1u));
-              if (at < out_end && at < d.contact_cap) d.c_col[at] = j;
-            }
-            out += __popc(bal);
-          }
-          __syncwarp(gm);
-          if (search && lane == 0) W.out[cc] = out;
-        }
       }
-      __syncwarp();
-      if (!FILL)
-        for (int a = l32; a < nc; a += 32) d.c_cnt[W.ci[a]] = W.pi[a] != -2 ? W.out[a] : 0;
     }
-    __syncwarp();  // the warp's stage is reused by the next cell
+    __syncwarp();
+    for (int o = LPN / 2; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    if (i >= 0 && sub == 0) d.c_cnt[i] = n;
   }
 }
 
@@ -889,8 +864,7 @@ __device__ void cand_cells(const DevData &d, uint8_t search_bit, CandWarp<DIM> *
 // writes the columns.  Lane t first takes neighbour cell t (empty when it
 // lies outside the grid or holds only nodes of this node's particle); the
 // cells' node ranges, concatenated in traversal order, are then walked 32
-// entries at a time, so each entry costs one chain of loads (its node, then
-// that node's particle and position) whatever cell it sits in.
+// entries at a time, two groups in flight.
 template <int DIM>
 __device__ void cand_fill_nodes(const DevData &d, int64_t nn) {
   constexpr int kNb = DIM == 3 ? 27 : 9;
@@ -901,14 +875,16 @@ __device__ void cand_fill_nodes(const DevData &d, int64_t nn) {
   const int64_t nwarps = (int64_t)gridDim.x * (kCoopBlock / 32);
   for (int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nn; t += nwarps) {
     const int32_t i = d.c_nodes[t];
+    const int2 sp = d.c_span[t];
     double q[3];
     ldv<DIM>(d.x, i, q);
     const int32_t pi = d.ptid[i];
-    int64_t out = d.c_row[i];
-    const int64_t out_end = d.c_row[i + 1];
-    for (int64_t e = out + l32; e < out_end && e < d.contact_cap; e += 32) d.c_own[e] = i;
-    const int cx0 = cell_coord<DIM>(q[0], G, 0), cy0 = cell_coord<DIM>(q[1], G, 1);
-    const int cz0 = DIM == 3 ? cell_coord<DIM>(q[2], G, 2) : 0;
+    const int cell0 = d.cell_of[i];
+    int64_t out = sp.x;
+    const int64_t out_end = min((int64_t)sp.y, d.contact_cap);
+    for (int64_t e = out + l32; e < out_end; e += 32) d.c_own[e] = i;
+    const int cx0 = cell0 % G.dims[0], cy0 = cell0 / G.dims[0] % G.dims[1];
+    const int cz0 = DIM == 3 ? cell0 / G.dims[0] / G.dims[1] : 0;
     int a = 0, cnt = 0;
     if (l32 < kNb) {
       const int cx = cx0 + l32 % 3 - 1, cy = cy0 + (l32 / 3) % 3 - 1, cz = DIM == 3 ? cz0 + l32 / 9 - 1 : 0;
@@ -929,35 +905,44 @@ __device__ void cand_fill_nodes(const DevData &d, int64_t nn) {
 #pragma unroll
     for (int c = 0; c < kNb; c++) inc[c] = __shfl_sync(0xffffffffu, incl, c);
     const int total = inc[kNb - 1];
-    for (int base = 0; base < total; base += 32) {
-      const int g = base + l32;
-      int k = 0;
+    for (int base = 0; base < total && out < out_end; base += 64) {
+      int at[2];
+      bool hit[2];
 #pragma unroll
-      for (int c = 0; c < kNb; c++) k += inc[c] <= g;
-      const int ak = __shfl_sync(0xffffffffu, a, k & 31);
-      const int ek = __shfl_sync(0xffffffffu, incl - cnt, k & 31);
-      bool hit = false;
-      int32_t j = -1;
-      if (g < total) {
-        j = d.cell_nodes[ak + (g - ek)];
-        if (d.ptid[j] != pi) {
-          double p[3];
-          ldv<DIM>(d.x, j, p);
+      for (int h = 0; h < 2; h++) {
+        const int g = base + 32 * h + l32;
+        int k = 0;
+#pragma unroll
+        for (int c = 0; c < kNb; c++) k += inc[c] <= g;
+        const int ak = __shfl_sync(0xffffffffu, a, k & 31);
+        const int ek = __shfl_sync(0xffffffffu, incl - cnt, k & 31);
+        at[h] = ak + (g - ek);
+        hit[h] = g < total;
+      }
+      int32_t pb[2] = {pi, pi};
+      double pos[2][3];
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        if (hit[h]) {
+          pb[h] = d.cell_p[at[h]];
+          ldv<DIM>(d.cell_x, at[h], pos[h]);
+        }
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        if (hit[h]) {
           double dd = 0.0;
 #pragma unroll
           for (int u = 0; u < DIM; u++) {
-            const double df = q[u] - p[u];
+            const double df = q[u] - pos[h][u];
             dd += df * df;
           }
-          hit = dd < r2;
+          hit[h] = pb[h] != pi && dd < r2;
         }
+        const unsigned bal = __ballot_sync(0xffffffffu, hit[h]);
+        const int64_t to = out + __popc(bal & ((1u << l32) - 1u));
+        if (hit[h] && to < out_end) d.c_col[to] = d.cell_nodes[at[h]];
+        out += __popc(bal);
       }
-      const unsigned bal = __ballot_sync(0xffffffffu, hit);
-      if (hit) {
-        const int64_t at = out + __popc(bal & ((1u << l32) - 1u));
-        if (at < out_end && at < d.contact_cap) d.c_col[at] = j;
-      }
-      out += __popc(bal);
     }
   }
 }
@@ -976,11 +961,9 @@ __device__ void list_live_tiles(const DevData &d) {
   }
 }
 
-template <int DIM, int LPN>
-__global__ void __launch_bounds__(kCoopBlock) k_contact_rebuild(DevData d, uint8_t search_bit,
-                                                               int64_t *bsum) {
-  extern __shared__ __align__(16) unsigned char cand_smem[];
-  CandWarp<DIM> *stage = reinterpret_cast<CandWarp<DIM> *>(cand_smem);
+template <int DIM>
+__global__ void __launch_bounds__(kCoopBlock, 4) k_contact_rebuild(const __grid_constant__ DevData d, uint8_t search_bit,
+                                                                  int64_t *bsum) {
   pdl_wait();
   if (d.ctrl->error) return;
   if (!d.ctrl->update) {
@@ -996,17 +979,13 @@ __global__ void __launch_bounds__(kCoopBlock) k_contact_rebuild(DevData d, uint8
     mark++;
   };
   stamp();
+  stamp();  // nothing to clear
   const int64_t nth = (int64_t)gridDim.x * blockDim.x;
   const int64_t N = d.n_nodes;
   const Grid G = d.grid;
-  for (int64_t c = tid; c <= G.ncells; c += nth) {
-    d.cell_cnt[c] = 0;
-    d.cell_fill[c] = 0;
-  }
+  // nodes per cell (the counters are zero between rebuilds)
   if (d.sur_near_gate)
     for (int64_t p = tid; p < d.n_particles; p += nth) d.sur_near[p] = 0;
-  if (!grid_bar(gc)) return;
-  stamp();
   for (int64_t i = tid; i < N; i += nth) {
     double p[3];
     ldv<DIM>(d.x, i, p);
@@ -1026,20 +1005,23 @@ __global__ void __launch_bounds__(kCoopBlock) k_contact_rebuild(DevData d, uint8
   if (!grid_bar(gc)) return;
   stamp();
   {
-    // per cell: its nodes in index order (rank counting) and, when they all
-    // belong to one particle, that particle (no candidate joins two nodes
-    // of one particle, so the searches skip a cell of the searching node's
-    // own particle)
+    // per cell: its nodes in index order (rank counting), their particles and
+    // positions in that order and, when they all belong to one particle, that
+    // particle; the counters back to zero
     const int lane = threadIdx.x & 31;
     for (int64_t c = tid >> 5; c < G.ncells; c += nth >> 5) {
       const int s = d.cell_start[c], e = d.cell_start[c + 1];
       int32_t pmin = INT32_MAX, pmax = -1;
       for (int a = s + lane; a < e; a += 32) {
         const int32_t va = d.cell_tmp[a];
+        const int32_t p = d.ptid[va];
+        double xa[3];
+        ldv<DIM>(d.x, va, xa);
         int rank = 0;
         for (int b = s; b < e; b++) rank += d.cell_tmp[b] < va;
         d.cell_nodes[s + rank] = va;
-        const int32_t p = d.ptid[va];
+        d.cell_p[s + rank] = p;
+        stv<DIM>(d.cell_x, s + rank, xa);
         pmin = min(pmin, p);
         pmax = max(pmax, p);
       }
@@ -1047,30 +1029,37 @@ __global__ void __launch_bounds__(kCoopBlock) k_contact_rebuild(DevData d, uint8
         pmin = min(pmin, __shfl_xor_sync(0xffffffffu, pmin, o));
         pmax = max(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
       }
-      if (lane == 0) d.cell_pid[c] = (e > s && pmin == pmax) ? pmin : -1;
+      if (lane == 0) {
+        d.cell_pid[c] = (e > s && pmin == pmax) ? pmin : -1;
+        d.cell_cnt[c] = 0;
+        d.cell_fill[c] = 0;
+      }
     }
   }
   if (!grid_bar(gc)) return;
   stamp();
-  cand_cells<DIM, LPN, false>(d, search_bit, stage);
+  cand_count<DIM, DIM == 2 ? kCandLanes2 : kCandLanes3>(d, search_bit);
   if (!grid_bar(gc)) return;
   stamp();
-  const int64_t *cn = d.c_cnt;
-  if (!grid_scan<int64_t>(gc, [cn](int64_t k) { return cn[k]; }, d.c_row, N, bsum)) return;
-  stamp();
-  if (!grid_scan<int64_t>(gc, [cn](int64_t k) { return (int64_t)(cn[k] > 0); }, d.c_tmp, N, bsum)) return;
-  stamp();
-  for (int64_t i = tid; i < N; i += nth)
-    if (cn[i] > 0) {
-      d.c_nodes[d.c_tmp[i]] = (int32_t)i;
-      d.c_span[d.c_tmp[i]] = make_int2((int)d.c_row[i], (int)d.c_row[i + 1]);
+  // row offsets and the compacted list of nodes with candidates
+  int64_t tot[2];
+  const bool ok = scan_rows(gc, d.c_cnt, N, bsum, tot, [&](int64_t i, int64_t cnt, int64_t row, int64_t at) {
+    d.c_row[i] = row;
+    if (cnt > 0) {
+      d.c_nodes[at] = (int32_t)i;
+      d.c_span[at] = make_int2((int)row, (int)(row + cnt));
       if (d.sur_near_gate) d.sur_near[d.ptid[i]] = 1;  // every writer stores the same value
     }
-  if (tid == 0) d.ctrl->c_nnodes = d.c_tmp[N];
-  if (!grid_bar(gc)) return;  // the compacted list is complete
-  list_live_tiles(d);          // the proximity flags are final
-  stamp();
-  cand_fill_nodes<DIM>(d, d.c_tmp[N]);
+  });
+  if (!ok) return;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+    d.c_row[N] = tot[0];
+    d.ctrl->c_nnodes = tot[1];
+  }
+  if (!grid_bar(gc)) return;
+  list_live_tiles(d);  // the proximity flags are final
+  for (int k = 0; k < 3; k++) stamp();  // row offsets, compaction offsets, lists: one pass
+  cand_fill_nodes<DIM>(d, d.ctrl->c_nnodes);
   stamp();  // the first CTA's share of the fill done
   if (tid == 0) {
     const int64_t total = d.c_row[N];
@@ -2155,9 +2144,8 @@ size_t scan_temp_bytes(int64_t n) {
 }
 
 
-template <int DIM, int LPN>
-static cudaError_t rebuild_dim(const DevData &d, uint8_t bit, int64_t *bsum, int grid,
-                               cudaStream_t s) {
+template <int DIM>
+static cudaError_t rebuild_dim(const DevData &d, uint8_t bit, int64_t *bsum, int grid, cudaStream_t s) {
   DevData dd = d;
   void *args[] = {(void *)&dd, (void *)&bit, (void *)&bsum};
   cudaLaunchAttribute at[2]{};
@@ -2168,31 +2156,29 @@ static cudaError_t rebuild_dim(const DevData &d, uint8_t bit, int64_t *bsum, int
   cudaLaunchConfig_t c{};
   c.gridDim = dim3(grid);
   c.blockDim = dim3(kCoopBlock);
-  c.dynamicSmemBytes = cand_stage_bytes<DIM>();
   c.stream = s;
   c.attrs = at;
   c.numAttrs = 2;
-  return cudaLaunchKernelExC(&c, (const void *)k_contact_rebuild<DIM, LPN>, args);
+  return cudaLaunchKernelExC(&c, (const void *)k_contact_rebuild<DIM>, args);
 }
 
-int rebuild_grid_blocks(const DevData &d, int lanes) {
+// Blocks of the cooperative rebuild: at most what is resident at once, and no
+// more than the nodes and cells keep busy (the whole
+// rebuild of a 634-node scene: 69 us with every resident block, 27 us with five)
+int rebuild_grid_blocks(const DevData &d) {
   int dev = 0, sms = 0, per = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const void *f;
-  if (d.dim == 2) f = lanes <= 8 ? (const void *)k_contact_rebuild<2, 8> : (const void *)k_contact_rebuild<2, 32>;
-  else f = lanes <= 8 ? (const void *)k_contact_rebuild<3, 8> : (const void *)k_contact_rebuild<3, 32>;
-  const size_t dyn = d.dim == 2 ? cand_stage_bytes<2>() : cand_stage_bytes<3>();
-  cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kCoopBlock, dyn);
-  return sms * (per > 0 ? per : 1);
+  const void *f = d.dim == 2 ? (const void *)k_contact_rebuild<2> : (const void *)k_contact_rebuild<3>;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f, kCoopBlock, 0);
+  const int64_t most = (int64_t)sms * (per > 0 ? per : 1);
+  const int64_t want = std::max<int64_t>((d.n_nodes + 127) / 128, ((int64_t)d.grid.ncells + 31) / 32);
+  return (int)std::min(most, want);
 }
 
-cudaError_t launch_contact_rebuild(const DevData &d, int64_t *bsum, int grid, int lanes, int init,
-                                   cudaStream_t s) {
+cudaError_t launch_contact_rebuild(const DevData &d, int64_t *bsum, int grid, int init, cudaStream_t s) {
   const uint8_t bit = init ? NODE_SEARCH0 : NODE_SEARCH;
-  if (d.dim == 2) return lanes <= 8 ? rebuild_dim<2, 8>(d, bit, bsum, grid, s) : rebuild_dim<2, 32>(d, bit, bsum, grid, s);
-  return lanes <= 8 ? rebuild_dim<3, 8>(d, bit, bsum, grid, s) : rebuild_dim<3, 32>(d, bit, bsum, grid, s);
+  return d.dim == 2 ? rebuild_dim<2>(d, bit, bsum, grid, s) : rebuild_dim<3>(d, bit, bsum, grid, s);
 }
 
 int sm_count() {

@@ -958,7 +958,6 @@ int prepare(pdgpu_ctx *ctx) {
   CK(cudaMemset(d.c_row, 0, ((size_t)N + 1) * 8));
   TRY(dalloc(ctx, &d.c_cnt, (size_t)N));
   CK(cudaMemset(d.c_cnt, 0, (size_t)N * 8));
-  TRY(dalloc(ctx, &d.c_tmp, (size_t)N + 1));
   TRY(dalloc(ctx, &d.c_nodes, (size_t)N));
   TRY(dalloc(ctx, &d.c_span, (size_t)N));
   CK(cudaMemset(d.c_span, 0, (size_t)N * sizeof(int2)));
@@ -1027,8 +1026,13 @@ int prepare(pdgpu_ctx *ctx) {
     if (!(cell > 0)) return fail(ctx, PDGPU_ERR_ARG, "max_contact_r must be positive");
     TRY(make_grid(ctx, cell, &g));
     TRY(ensure_cells(ctx, g));
-    ctx->rebuild_grid = rebuild_grid_blocks(d, ctx->contact_lanes);
-    TRY(dalloc(ctx, &ctx->rebuild_bsum, (size_t)ctx->rebuild_grid + 1));
+    // the rebuild finds its cell counters at zero and leaves them so
+    CK(cudaMemset(d.cell_cnt, 0, ((size_t)g.ncells + 1) * 4));
+    CK(cudaMemset(d.cell_fill, 0, ((size_t)g.ncells + 1) * 4));
+    TRY(dalloc(ctx, &d.cell_p, (size_t)N));
+    TRY(dalloc(ctx, &d.cell_x, (d.dim == 2 ? 2 : 4) * (size_t)N));
+    ctx->rebuild_grid = rebuild_grid_blocks(d);
+    TRY(dalloc(ctx, &ctx->rebuild_bsum, 2 * (size_t)ctx->rebuild_grid));
   }
   // step control
   CtrlState c{};
@@ -1132,7 +1136,7 @@ void compute_forces(pdgpu_ctx *ctx, bool step) {
   if (ctx->desc.multi_particle) {
     // the cooperative rebuild stays on the main stream, ahead of the fork
     run(ctx, "contact_update", [&] {
-      launch_contact_rebuild(d, ctx->rebuild_bsum, ctx->rebuild_grid, ctx->contact_lanes, 0, s);
+      launch_contact_rebuild(d, ctx->rebuild_bsum, ctx->rebuild_grid, 0, s);
     });
     cudaEventRecord(ctx->ev_fork, s);
     cudaStreamWaitEvent(ctx->branch, ctx->ev_fork, 0);
@@ -1184,7 +1188,7 @@ cudaError_t graph_step(pdgpu_ctx *ctx, const char **where) {
     // at once on steps without a rebuild; on the main path, where nothing
     // else runs beside its grid-wide syncs
     *where = "contact-list rebuild";
-    e = launch_contact_rebuild(d, ctx->rebuild_bsum, ctx->rebuild_grid, ctx->contact_lanes, 0, s);
+    e = launch_contact_rebuild(d, ctx->rebuild_bsum, ctx->rebuild_grid, 0, s);
     if (e != cudaSuccess) return e;
     // branch (captured first, so its kernels are dispatched ahead of the bond
     // loop's tiles): contact forces, then damping
@@ -1630,7 +1634,7 @@ int pdgpu_init_contact(pdgpu_ctx *ctx) {
   if (!ctx->desc.multi_particle) return PDGPU_OK;
   if (ctx->contact_init) return fail(ctx, PDGPU_ERR_STATE, "contact lists already initialised");
   launch_ctrl(ctx->d, 2, ctx->stream);
-  CK(launch_contact_rebuild(ctx->d, ctx->rebuild_bsum, ctx->rebuild_grid, ctx->contact_lanes, 1,
+  CK(launch_contact_rebuild(ctx->d, ctx->rebuild_bsum, ctx->rebuild_grid, 1,
                             ctx->stream));
   // no bond loop follows this rebuild: clear the surrogate's tile list
   if (ctx->d.tile_live) CK(cudaMemsetAsync(ctx->d.tile_live_n, 0, 4, ctx->stream));
