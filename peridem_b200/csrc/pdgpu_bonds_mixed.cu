@@ -582,9 +582,8 @@ __device__ __forceinline__ void tile_sym(const DevData &d, const BondTile &T, co
   }
 }
 
-// Persistent: a fixed grid (below full occupancy, so that the contact and
-// damping passes running beside it find room) claims tiles from a counter in
-// the step-control state; the claim for the next tile is made while the
+// Persistent: a fixed grid claims tiles from a counter in the step-control
+// state; the claim for the next tile is made while the
 // current one is staged.  The last CTA out resets the counter.
 template <int DIM, int LPN, int LAW, typename CT, bool PRE = false, bool SYM = false>
 __global__ void __launch_bounds__(kThreadsFor<DIM, LPN>) k_bonds_mixed(DevData d, const BondTile *tiles, int n_tiles,
@@ -695,10 +694,13 @@ __global__ void __launch_bounds__(kThreadsFor<DIM, LPN>) k_bonds_mixed(DevData d
   }
 }
 
-// CTAs per SM for the persistent bond loop: one below the occupancy limit
-// (the occupancy limit itself when it is two or less)
+// CTAs per SM for the persistent bond loop: the occupancy limit (the contact
+// pass is placed ahead of it); with the learned surrogate, whose chain runs on a
+// third stream beside it, one less where at least three fit.  (One slot left
+// free for all: 332 000 nodes 49.3 us a step against 48.5, 1.3 M nodes 160.8
+// against 154.2.)
 template <class K>
-int bond_grid(K kernel, int threads, size_t smem, int n_tiles) {
+int bond_grid(K kernel, int threads, size_t smem, int n_tiles, bool surrogate) {
   static int sms = 0;
   if (!sms) {
     int dev = 0;
@@ -708,9 +710,7 @@ int bond_grid(K kernel, int threads, size_t smem, int n_tiles) {
   }
   int per = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
-  // one slot per SM stays free for the contact and damping passes when at
-  // least three fit; with two, both go to the bond loop
-  const int g = sms * (per > 2 ? per - 1 : (per > 0 ? per : 1));
+  const int g = sms * (surrogate && per > 2 ? per - 1 : (per > 0 ? per : 1));
   return g < n_tiles ? g : n_tiles;
 }
 
@@ -718,7 +718,7 @@ template <int DIM, int LPN, int LAW, typename CT, bool PRE = false, bool SYM = f
 void launch_one(const DevData &d, const CT *col, const BondTile *t, int n, size_t smem, cudaStream_t s) {
   auto *k = k_bonds_mixed<DIM, LPN, LAW, CT, PRE, SYM>;
   constexpr int kT = kThreadsFor<DIM, LPN>;
-  const int g = bond_grid(k, kT, smem, n);
+  const int g = bond_grid(k, kT, smem, n, d.sur_on != nullptr);
   // in 3-D k_urel, the pre-pass or another law's launch is ahead; in 2-D the
   // contact rebuild may be, and CTAs that came before the contact pass's
   // would leave those no room
