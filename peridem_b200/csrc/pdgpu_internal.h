@@ -162,6 +162,14 @@ struct SurPart {
   double c, s, inv_scale, fscale, floor2;
 };
 
+// what the post-processing of a test-output step reads of the positions before
+// the next step has moved them (k_step_turn): the test wall's first node, the
+// first two particles' centres, the second one's largest y (as an ordered key)
+struct TurnState {
+  double wall[3], centre[2][3];
+  unsigned long long max_y;
+};
+
 struct DevData {
   int32_t dim;
   int32_t precision;
@@ -255,6 +263,7 @@ struct DevData {
   int32_t cr_blocks;
 
   CtrlState *ctrl;
+  TurnState *turn;
 
   // mixed-precision bond loop: particle-local FP32 reference coordinates,
   // FP32 volumes, particle-local 16-bit neighbour offsets when they fit
@@ -390,6 +399,10 @@ void launch_ctrl(const DevData &d, int mode, cudaStream_t s);  // mode 0 step, 1
 void launch_step_begin(const DevData &d, int verlet, cudaStream_t s);
 // external forces + force BC (+ Verlet second half) + post-processing (last CTA)
 void launch_step_end(const DevData &d, int verlet, int post, cudaStream_t s);
+// step end of one step and step begin of the next, in one kernel (scenes up
+// to kTurnMaxNodes nodes)
+constexpr int64_t kTurnMaxNodes = 148 * 4 * 256;
+void launch_step_turn(const DevData &d, int verlet, cudaStream_t s);
 void launch_bc(const DevData &d, cudaStream_t s);
 void launch_mixed_setup(const DevData &d, cudaStream_t s);
 // symmetric layout: per node its tile (node_tile) -> counts (n_up, n_uo into

@@ -1740,11 +1740,23 @@ __global__ void k_force_bc(const __grid_constant__ DevData d) {
 // Post-processing every test_interval steps: DEMModel::ppCompressiveTest
 // (demModel.cpp:2202-2250) or ppTwoParticleTest (:2096-2149).
 // ---------------------------------------------------------------------------
+// doubles as unsigned keys of the same order (0 below every key)
+__device__ __forceinline__ unsigned long long to_key(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  return b >> 63 ? ~b : b | (1ull << 63);
+}
+__device__ __forceinline__ double from_key(unsigned long long k) {
+  if (k == 0) return -DBL_MAX;  // no value
+  return __longlong_as_double((long long)(k >> 63 ? k & ~(1ull << 63) : ~k));
+}
+
 // The test's post-processing (demModel.cpp ppCompressiveTest / ppTwoParticleTest)
 // run by one 1024-thread block; forces of the current step are read past L1,
 // since other CTAs of the same kernel may have written them.
+// pre: the positions it needs, where the caller has moved the nodes on already
+// (TurnState; null: they are in d.x)
 template <int DIM>
-__device__ __noinline__ void postprocess_block(const DevData &d) {
+__device__ __noinline__ void postprocess_block(const DevData &d, const TurnState *pre = nullptr) {
   // sums are formed as by a 1024-thread block (per-thread strided partials,
   // warp butterflies, then the 32 warp sums in order), whatever blockDim is
   constexpr int kV = 1024;
@@ -1778,7 +1790,7 @@ __device__ __noinline__ void postprocess_block(const DevData &d) {
         rs += red[0][w];
         rc += red[1][w];
       }
-      const double delta = d.x[st * W.start + dir] - d.xref[st * W.start + dir];
+      const double delta = (pre ? pre->wall[dir] : d.x[st * W.start + dir]) - d.xref[st * W.start + dir];
       c->reaction = rs;
       c->contact_reaction = -rc;
       c->penetration = delta;
@@ -1793,7 +1805,7 @@ __device__ __noinline__ void postprocess_block(const DevData &d) {
     }
   } else if (d.test == PDGPU_TEST_TWO_PARTICLE && d.n_particles >= 2) {
     const DevParticle P0 = d.particles[0], P1 = d.particles[1];
-    for (int vt = threadIdx.x; vt < kV; vt += blockDim.x) {
+    for (int vt = threadIdx.x; vt < kV && !pre; vt += blockDim.x) {
       double m = -DBL_MAX;
       for (int64_t i = P1.start + vt; i < P1.end; i += kV) m = fmax(m, d.x[st * i + 1]);
       for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -1801,10 +1813,11 @@ __device__ __noinline__ void postprocess_block(const DevData &d) {
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-      double my = -DBL_MAX;
-      for (int w = 0; w < kV / 32; w++) my = fmax(my, red[0][w]);
+      double my = pre ? from_key(pre->max_y) : -DBL_MAX;
+      for (int w = 0; w < kV / 32 && !pre; w++) my = fmax(my, red[0][w]);
       double dx[3] = {0, 0, 0};
-      for (int q = 0; q < DIM; q++) dx[q] = d.x[st * P1.center + q] - d.x[st * P0.center + q];
+      for (int q = 0; q < DIM; q++)
+        dx[q] = pre ? pre->centre[1][q] - pre->centre[0][q] : d.x[st * P1.center + q] - d.x[st * P0.center + q];
       const double r = P0.bound_r;
       const ContactPair cp = d.contact[P0.zone * d.n_zones + P1.zone];
       const double re = r + cp.rc;
@@ -1981,6 +1994,153 @@ __global__ void __launch_bounds__(kBlock) k_step_end(const __grid_constant__ Dev
     __threadfence();
     if (threadIdx.x == 0) d.ctrl->end_done = 0u;
     postprocess_block<DIM>(d);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Between two steps of a graph: the last kernel of one step (k_step_end) and
+// the first of the next (k_step_begin) in one pass over the nodes, with their
+// operations in their order: f is written but not read again, node constants
+// and control state are read once, and a launch goes.  On test-output steps
+// the positions the post-processing needs go to d.turn before they move on;
+// the last CTA runs it, then the step control.
+//
+// For scenes up to a wave of CTAs (kTurnMaxNodes), where the two kernels are a
+// chain of latencies: us per step without / with it, two discs FP64 14.8 / 13.1,
+// PMB with Verlet 18.5 / 15.7, 24 000 nodes 26.4 / 24.9.  Larger ones gain
+// nothing (332 000 nodes 49.2 / 49.2 to 50.0, 1.3 M 154.1 / 152.8 to 158.7 over
+// one or two nodes per thread, bulk prefetch of later CTAs' nodes 156.5; 3-D,
+// 244 000 nodes 142.8 / 144.4): the traffic saved is a tenth, and the longer
+// kernel holds fewer warps.
+// ---------------------------------------------------------------------------
+template <int DIM, bool VERLET>
+__global__ void __launch_bounds__(kBlock) k_step_turn(const __grid_constant__ DevData d) {
+  __shared__ double smax[kBlock / 32];
+  __shared__ int last;
+  __shared__ __align__(8) CtrlState s_ctrl;
+  pdl_start();
+  if (threadIdx.x < sizeof(CtrlState) / 8)
+    reinterpret_cast<uint64_t *>(&s_ctrl)[threadIdx.x] = reinterpret_cast<const uint64_t *>(d.ctrl)[threadIdx.x];
+  const int64_t n_step = d.ctrl->n;
+  const double time = d.ctrl->time;
+  const bool post = d.test != PDGPU_TEST_NONE && n_step % d.test_interval == 0 && n_step >= d.test_interval;
+  // reverse node order, as step begin
+  const int64_t i = (int64_t)(gridDim.x - 1 - blockIdx.x) * kBlock + threadIdx.x;
+  double vm = 0.0;
+  unsigned long long ymax = 0;
+  if (!d.ctrl->error && i < d.n_nodes) {
+    double v[3], u[3], x[3], f[3];
+    const uint8_t fl = d.flags[i], fix = d.fix[i];
+    const int32_t pid = d.ptid[i];
+    ldv<DIM>(d.f, i, f);
+    ldv<DIM>(d.v, i, v);
+    ldv<DIM>(d.u, i, u);
+    ldv<DIM>(d.x, i, x);
+    const bool active = fl & NODE_ACTIVE;
+    const double rho = d.particles[pid].density;
+    // ---- end of the step (k_step_end)
+    if (!active) f[0] = f[1] = f[2] = 0.0;
+    if (active && d.fc && (fl & (NODE_SEARCH | NODE_SEARCH0))) {
+      double c[3];
+      ldv<DIM>(d.fc, i, c);
+      if (c[0] != 0.0 || c[1] != 0.0 || (DIM == 3 && c[2] != 0.0)) {
+#pragma unroll
+        for (int q = 0; q < DIM; q++) f[q] += c[q];
+        const double z[3] = {0.0, 0.0, 0.0};
+        stv<DIM>(d.fc, i, z);
+      }
+    }
+    if (fl & NODE_PARTICLE) {
+#pragma unroll
+      for (int q = 0; q < DIM; q++) f[q] += d.fdamp[4 * pid + q];
+    }
+    if (d.gravity_on) {
+#pragma unroll
+      for (int q = 0; q < DIM; q++) f[q] += rho * d.gravity[q];
+    }
+    if (fl & NODE_FBC) {  // through a copy, so that f stays in registers
+      double fb[3] = {f[0], f[1], f[2]};
+      apply_fbc<DIM>(d, d.fbc_of[i], time, fb);
+#pragma unroll
+      for (int q = 0; q < 3; q++) f[q] = fb[q];
+    }
+    stv<DIM>(d.f, i, f);
+    if (post) {
+      TurnState *t = d.turn;
+      if (d.test == PDGPU_TEST_COMPRESSIVE) {
+        if (i == d.particles[d.test_wall].start)
+          for (int q = 0; q < DIM; q++) t->wall[q] = x[q];
+      } else if (d.n_particles >= 2 && pid <= 1) {
+        if (i == d.particles[pid].center)
+          for (int q = 0; q < DIM; q++) t->centre[pid][q] = x[q];
+        if (pid == 1 && x[1] == x[1]) ymax = to_key(x[1]);
+      }
+    }
+    // ---- begin of the next (k_step_begin)
+    if (fl & (NODE_ACTIVE | NODE_UBC)) {
+      if (active) {
+        const double dt = d.dt;
+        const double kk = VERLET ? 0.5 * (dt / rho) : dt / rho;
+#pragma unroll
+        for (int dof = 0; dof < DIM; dof++) {
+          if (!((fix >> dof) & 1u)) {
+            if (VERLET) v[dof] += kk * f[dof];  // the ended step's second half
+            v[dof] += kk * f[dof];
+            u[dof] += dt * v[dof];
+            x[dof] += dt * v[dof];
+          }
+        }
+        vm = len3<DIM>(v);
+        d.vmag[i] = vm;
+      }
+      if (fl & NODE_UBC) {
+        double ub[3], vb[3], xb[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++) ub[q] = u[q], vb[q] = v[q], xb[q] = x[q];
+        apply_ubc<DIM>(d, d.ubc_of[i], i, time + d.dt, 0, ub, vb, xb);
+#pragma unroll
+        for (int q = 0; q < 3; q++) u[q] = ub[q], v[q] = vb[q], x[q] = xb[q];
+      }
+      stv<DIM>(d.v, i, v);
+      stv<DIM>(d.u, i, u);
+      stv<DIM>(d.x, i, x);
+    }
+  }
+  if (post && d.test == PDGPU_TEST_TWO_PARTICLE && ymax) atomicMax(&d.turn->max_y, ymax);
+  // block max of |v| -> one atomic per block
+  for (int o = 16; o > 0; o >>= 1) vm = fmax(vm, __shfl_xor_sync(0xffffffffu, vm, o));
+  if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = vm;
+  if (post) __threadfence();  // this thread's f and d.turn, for the last CTA
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    double m = threadIdx.x < kBlock / 32 ? smax[threadIdx.x] : 0.0;
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (threadIdx.x == 0) {
+      if (m > 0.0) atomic_max_nonneg(&d.ctrl->vmax_bits, m);
+      __threadfence();
+      last = atomicAdd(&d.ctrl->begin_done, 1u) == gridDim.x - 1;
+    }
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (post) {
+    __shared__ TurnState s_turn;
+    if (threadIdx.x == 0) {
+      for (int q = 0; q < 3; q++) {
+        s_turn.wall[q] = __ldcg(d.turn->wall + q);
+        s_turn.centre[0][q] = __ldcg(d.turn->centre[0] + q);
+        s_turn.centre[1][q] = __ldcg(d.turn->centre[1] + q);
+      }
+      s_turn.max_y = atomicExch(&d.turn->max_y, 0ull);
+    }
+    __syncthreads();
+    postprocess_block<DIM>(d, &s_turn);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    d.ctrl->begin_done = 0u;
+    ctrl_step(d, 0, &s_ctrl);
   }
 }
 
@@ -2255,6 +2415,17 @@ void launch_step_end(const DevData &d, int verlet, int post, cudaStream_t s) {
   } else {
     if (verlet) k_step_end<3, true><<<g, kBlock, 0, s>>>(d, post);
     else k_step_end<3, false><<<g, kBlock, 0, s>>>(d, post);
+  }
+}
+
+void launch_step_turn(const DevData &d, int verlet, cudaStream_t s) {
+  const unsigned g = blocks_for(d.n_nodes, kBlock);
+  if (d.dim == 2) {
+    if (verlet) k_step_turn<2, true><<<g, kBlock, 0, s>>>(d);
+    else k_step_turn<2, false><<<g, kBlock, 0, s>>>(d);
+  } else {
+    if (verlet) k_step_turn<3, true><<<g, kBlock, 0, s>>>(d);
+    else k_step_turn<3, false><<<g, kBlock, 0, s>>>(d);
   }
 }
 

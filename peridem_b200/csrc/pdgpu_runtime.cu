@@ -1034,6 +1034,8 @@ int prepare(pdgpu_ctx *ctx) {
     ctx->rebuild_grid = rebuild_grid_blocks(d);
     TRY(dalloc(ctx, &ctx->rebuild_bsum, 2 * (size_t)ctx->rebuild_grid));
   }
+  TRY(dalloc(ctx, &d.turn, 1));
+  CK(cudaMemset(d.turn, 0, sizeof *d.turn));
   // step control
   CtrlState c{};
   c.interval = ctx->desc.search_interval;
@@ -1174,14 +1176,17 @@ void one_step(pdgpu_ctx *ctx) {
   compute_forces(ctx, true);
 }
 
-// One step inside a graph under capture: the same kernels as one_step,
-// captured without the timing events.
-cudaError_t graph_step(pdgpu_ctx *ctx, const char **where) {
+// One step inside a graph under capture: the same kernels as one_step, captured
+// without the timing events; `begin` and `end`: with its first and last kernel.
+// Between two steps of a graph of a small scene one kernel does both
+// (launch_step_turn), except in an ensemble, whose test output reads the state in
+// between.
+cudaError_t graph_step(pdgpu_ctx *ctx, const char **where, bool begin, bool end) {
   DevData &d = ctx->d;
   cudaStream_t s = ctx->stream;
   const bool verlet = ctx->desc.time_scheme == 1;
   const bool mixed = d.precision == PDGPU_PREC_MIXED;
-  launch_step_begin(d, verlet ? 1 : 0, s);
+  if (begin) launch_step_begin(d, verlet ? 1 : 0, s);
   cudaError_t e = cudaSuccess;
   if (ctx->desc.multi_particle) {
     // contact-list rebuild: the single-launch cooperative kernel, which exits
@@ -1233,8 +1238,12 @@ cudaError_t graph_step(pdgpu_ctx *ctx, const char **where) {
     if (e != cudaSuccess) return e;
   }
   *where = "kernels after the join";
-  launch_step_end(d, verlet ? 1 : 0, 1, s);
-  launch_scene_post(d, s);
+  if (end) {
+    launch_step_end(d, verlet ? 1 : 0, 1, s);
+    launch_scene_post(d, s);
+  } else {
+    launch_step_turn(d, verlet ? 1 : 0, s);
+  }
   return cudaGetLastError();
 }
 
@@ -1245,7 +1254,8 @@ int build_graph(pdgpu_ctx *ctx, int steps) {
   const char *where = "graph_step";
   cudaError_t e = cudaSuccess;
   int k = 0;
-  for (; k < steps && e == cudaSuccess; k++) e = graph_step(ctx, &where);
+  const bool turns = ctx->d.n_scenes <= 1 && ctx->d.n_nodes <= kTurnMaxNodes;
+  for (; k < steps && e == cudaSuccess; k++) e = graph_step(ctx, &where, k == 0 || !turns, k + 1 == steps || !turns);
   const cudaError_t e2 = cudaStreamEndCapture(s, &g);
   if (e != cudaSuccess || e2 != cudaSuccess) {
     if (g) cudaGraphDestroy(g);
