@@ -30,9 +30,10 @@
 //   FP64 and 83 other thread instructions per bond; 40 us of FP64 issue);
 //   3-D, PD state, 75 000 sphere nodes, 6.5 M bonds: pre-pass 126 -> 54, main
 //   loop 337 -> 69; 3-D, PD elastic, 64 000 sphere nodes: 304 -> 55.
-// The outputs are the same to the bit at equal lanes per node.  Three CTAs of
-// 256 threads per SM (80 registers) in 2-D: 84 us where two (114 registers)
-// take 116 and four (64 registers, spills) 81 alone but 2 us more per step.
+// The outputs are the same to the bit at equal lanes per node.  Four CTAs of
+// 256 threads per SM in 2-D (64 registers, 30 to 60 bytes of spills): a step of
+// the 333 000-node compression takes 91.8 us, with three (80 registers) 94.5;
+// with two (114 registers) the launch alone took a third longer.
 #include <cfloat>
 #include <cstdint>
 #include <type_traits>
@@ -299,7 +300,7 @@ __device__ __forceinline__ bool bond64(const Bond64<DIM> &B, const Node64 &I, in
 // whose window leaves no room, and reference distances outside the range of
 // the unchecked root).
 template <int DIM, int LPN, int LAW, bool PRE, typename COL>
-__global__ void __launch_bounds__(kThreads64<DIM>, DIM == 2 ? 3 : 1)
+__global__ void __launch_bounds__(kThreads64<DIM>, DIM == 2 ? 4 : 1)
     k_bonds_fp64(const __grid_constant__ DevData d, const BondTile *__restrict__ tiles, int stage) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar;
