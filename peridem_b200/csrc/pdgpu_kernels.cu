@@ -1844,6 +1844,8 @@ template <int DIM>
 __global__ void __launch_bounds__(256) k_scene_post(const __grid_constant__ DevData d) {
   __shared__ double red[2][8];
   __shared__ int64_t range[2];
+  pdl_start();
+  pdl_wait();
   const CtrlState *c = d.ctrl;
   if (c->error) return;
   const int64_t n = c->n;
@@ -2385,8 +2387,7 @@ void launch_contact_force(const DevData &d, int lanes, cudaStream_t s) {
 
 void launch_scene_post(const DevData &d, cudaStream_t s) {
   if (d.n_scenes <= 1) return;
-  if (d.dim == 2) k_scene_post<2><<<d.n_scenes, 256, 0, s>>>(d);
-  else k_scene_post<3><<<d.n_scenes, 256, 0, s>>>(d);
+  launch_dependent(d.dim == 2 ? k_scene_post<2> : k_scene_post<3>, d.n_scenes, 256, 0, s, d);
 }
 
 void launch_damping(const DevData &d, cudaStream_t s) {
