@@ -66,7 +66,7 @@ struct pdgpu_ctx {
   void *scan_tmp = nullptr;
   size_t scan_bytes = 0;
   int pd_lanes = 0, contact_lanes = 1;
-  int contact_ctas = 2;  // CTAs per SM of the contact node pass (two fit beside the bond loop)
+  int contact_ctas = 0;  // CTAs per SM of the contact node pass (0: by the scene's size)
   int64_t *rebuild_bsum = nullptr;
   int rebuild_grid = 0;
   // tiled bond loop
@@ -679,7 +679,7 @@ void choose_tiling(pdgpu_ctx *ctx) {
   if (ctx->pd_lanes <= 0) ctx->pd_lanes = lanes0;
   if (choose) {
     const int threads = d.dim == 3 ? 512 : (mixed ? 128 : 256);
-    const int64_t room = (int64_t)sm_count() * (d.dim == 2 ? 3 : 1);  // FP64 CTAs at once
+    const int64_t room = (int64_t)sm_count() * (d.dim == 2 ? 4 : 1);  // FP64 CTAs at once
     int64_t active = 0;
     for (const auto &P : ctx->hp) active += P.compute_force ? P.end - P.start : 0;
     for (int l = 2 * lanes0; !mixed && l <= 16 && l <= bpn; l *= 2) {
@@ -928,9 +928,13 @@ int prepare(pdgpu_ctx *ctx) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // four CTAs per SM: the pass is bound by the latency of its gathers (a
-    // cold L2 after every step), so it wants many candidates in flight; the
-    // CTAs that find no free slot beside the bond loop start as it drains
+    // Two CTAs per SM, one in scenes of medium size: the bond loop's first
+    // CTAs wait for the contact pass's, so where one CTA per SM gets through
+    // the candidates quickly the bond loop starts earlier (us per step with one
+    // / two: 332 000 nodes FP32 form 48.0 / 49.4, FP64 90.0 / 91.8, an ensemble
+    // of 416 000 55.1 / 56.0; but 24 000 nodes 25.0 / 23.7, where the pass is
+    // the longest chain beside a short bond loop, and 1.3 M 155.9 / 154.3)
+    if (ctx->contact_ctas <= 0) ctx->contact_ctas = N > kTurnMaxNodes && N <= 4 * kTurnMaxNodes ? 1 : 2;
     d.contact_grid = ctx->contact_ctas * (sms > 0 ? sms : 148);
   }
   d.cr_blocks = d.contact_grid;
