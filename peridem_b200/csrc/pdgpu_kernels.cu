@@ -2362,8 +2362,23 @@ void launch_contact_force(const DevData &d, int lanes, cudaStream_t s) {
   const unsigned g = (unsigned)d.contact_grid;
   if (lanes == 1) {  // one kernel, a warp per 32 nodes
     const unsigned gc = g + blocks_for(d.n_particles, kBlock / 32);
-    if (d.dim == 2) k_contact_warp<2><<<gc, kBlock, 0, s>>>(d);
-    else k_contact_warp<3><<<gc, kBlock, 0, s>>>(d);
+    // In front of the FP32 2-D bond loop (150 KB of shared memory per SM over its
+    // ten CTAs) the pass asks for the same carve-out, since an SM changes its
+    // carve-out only when empty: the bond loop's CTAs then start beside the
+    // contact pass's.  us per step without / with: two discs 14.7 / 14.5, 24 000
+    // nodes 22.9 / 21.5, 332 000 47.9 / 47.7, an ensemble of 416 000 55.3 / 55.3.
+    // Not for 1.3 M nodes, where the pass wants its L1 (154.0 / 154.9), nor before
+    // the FP64 loop (88.8 / 90.0).
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    at.val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3(gc);
+    c.blockDim = dim3(kBlock);
+    c.stream = s;
+    c.attrs = &at;
+    c.numAttrs = d.precision == PDGPU_PREC_MIXED && d.dim == 2 && d.n_nodes <= 4 * kTurnMaxNodes ? 1 : 0;
+    cudaLaunchKernelEx(&c, d.dim == 2 ? k_contact_warp<2> : k_contact_warp<3>, d);
     return;
   }
   PDGPU_DIM_DISPATCH(d, k_damp_pairs, <<<blocks_for(d.n_particles, kBlock / 32), kBlock, 0, s>>>(d));
