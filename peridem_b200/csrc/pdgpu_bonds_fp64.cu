@@ -471,13 +471,15 @@ __global__ void k_fp64_setup(const __grid_constant__ DevData d) {
   d.fa[i] = make_double2((3. * P.mat[0] / m) - a / 3., a);
 }
 
-// any reference distance of the lists outside root_in_range's range?
+// any reference distance of the lists outside root_in_range's range? (a warp
+// per node: its list is contiguous)
 __global__ void k_fp64_range(const __grid_constant__ DevData d, int32_t *outside) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (i >= d.n_nodes) return;
   const int st = d.dim == 2 ? 2 : 4;
+  const int64_t e = d.pd_row[i + 1];
   bool out = false;
-  for (int64_t k = d.pd_row[i]; k < d.pd_row[i + 1]; k++) {
+  for (int64_t k = d.pd_row[i] + (threadIdx.x & 31); k < e; k += 32) {
     double r2 = 0.0;
     for (int q = 0; q < d.dim; q++) {
       const double dx = d.xref[st * (int64_t)d.pd_col[k] + q] - d.xref[st * i + q];
@@ -547,7 +549,7 @@ void launch_fp64_setup(const DevData &d, cudaStream_t s) {
 }
 
 void launch_fp64_range(const DevData &d, int32_t *outside, cudaStream_t s) {
-  k_fp64_range<<<(unsigned)((d.n_nodes + 255) / 256), 256, 0, s>>>(d, outside);
+  k_fp64_range<<<(unsigned)((d.n_nodes + 7) / 8), 256, 0, s>>>(d, outside);
 }
 
 void launch_pd_tiled_fp64(const DevData &d, const BondTile *t, const int *law_begin, int lanes, int stage,

@@ -43,19 +43,20 @@ __global__ void k_tile_windows(DevData d, BondTile *tiles) {
   }
 }
 
-__global__ void k_mixed_setup(DevData d) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_mixed_setup(const __grid_constant__ DevData d) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // a warp per node: its list is contiguous
+  const int lane = threadIdx.x & 31;
   if (i >= d.n_nodes) return;
   const DevParticle &P = d.particles[d.ptid[i]];
-  if (d.xv_mixed) {  // mixed form
+  if (d.xv_mixed && lane == 0) {  // mixed form
     const int st = d.dim == 2 ? 2 : 4;
     float r[3] = {0.f, 0.f, 0.f};
     for (int q = 0; q < d.dim; q++) r[q] = (float)(d.xref[st * i + q] - d.xref[st * P.center + q]);
     d.xv_mixed[i] = make_float4(r[0], r[1], r[2], (float)d.vol[i]);
   }
   if (!d.use16) return;
-  for (int64_t k = d.pd_row[i]; k < d.pd_row[i + 1]; k++)
-    d.pd_col16[k] = (uint16_t)(d.pd_col[k] - P.start);
+  const int64_t e = d.pd_row[i + 1];
+  for (int64_t k = d.pd_row[i] + lane; k < e; k += 32) d.pd_col16[k] = (uint16_t)(d.pd_col[k] - P.start);
 }
 
 // Symmetric layout, pass 1: per node of a tile, how many of its bonds go to
@@ -181,7 +182,7 @@ void launch_tile_windows(const DevData &d, BondTile *tiles, int n_tiles, cudaStr
 }
 
 void launch_mixed_setup(const DevData &d, cudaStream_t s) {
-  k_mixed_setup<<<(unsigned)((d.n_nodes + 255) / 256), 256, 0, s>>>(d);
+  k_mixed_setup<<<(unsigned)((d.n_nodes + 7) / 8), 256, 0, s>>>(d);
 }
 
 }  // namespace pdgpu

@@ -1022,9 +1022,11 @@ int prepare(pdgpu_ctx *ctx) {
     TRY(dalloc(ctx, &d.wp, ctx->hp.size() * (size_t)d.wp_cap));
     TRY(dalloc(ctx, &d.wp_cnt, ctx->hp.size()));
     CK(cudaMemset(d.wp_cnt, 0, ctx->hp.size() * 4));
-    TRY(dalloc(ctx, &d.cell_of, N));
-    TRY(dalloc(ctx, &d.cell_tmp, N));
-    TRY(dalloc(ctx, &d.cell_nodes, N));
+    // (there already where the bond lists were built on the device; an
+    // allocation of this size costs 0.2-0.4 ms)
+    if (!d.cell_of) TRY(dalloc(ctx, &d.cell_of, N));
+    if (!d.cell_tmp) TRY(dalloc(ctx, &d.cell_tmp, N));
+    if (!d.cell_nodes) TRY(dalloc(ctx, &d.cell_nodes, N));
     Grid g{};
     const double cell = std::max(1.0, ctx->desc.search_factor) * ctx->desc.max_contact_r;
     if (!(cell > 0)) return fail(ctx, PDGPU_ERR_ARG, "max_contact_r must be positive");
@@ -1033,8 +1035,9 @@ int prepare(pdgpu_ctx *ctx) {
     // the rebuild finds its cell counters at zero and leaves them so
     CK(cudaMemset(d.cell_cnt, 0, ((size_t)g.ncells + 1) * 4));
     CK(cudaMemset(d.cell_fill, 0, ((size_t)g.ncells + 1) * 4));
-    TRY(dalloc(ctx, &d.cell_p, (size_t)N));
-    TRY(dalloc(ctx, &d.cell_x, (d.dim == 2 ? 2 : 4) * (size_t)N));
+    const size_t sx = (d.dim == 2 ? 2 : 4) * (size_t)N;
+    TRY(dalloc(ctx, &d.cell_x, sx + (size_t)(N + 1) / 2));
+    d.cell_p = reinterpret_cast<int32_t *>(d.cell_x + sx);  // N of them behind the positions
     ctx->rebuild_grid = rebuild_grid_blocks(d);
     TRY(dalloc(ctx, &ctx->rebuild_bsum, 2 * (size_t)ctx->rebuild_grid));
   }
