@@ -486,6 +486,11 @@ PDGPU_API int pdgpu_write_strain_vtu(pdgpu_ctx *ctx, const char *path, int64_t n
 PDGPU_API int pdgpu_enable_rebuild_phases(pdgpu_ctx *ctx, int32_t on);
 PDGPU_API int pdgpu_rebuild_phases(pdgpu_ctx *ctx, int64_t *ns, int32_t cap, int32_t *count);
 
+/* Longest wait, in ns, of a block at a grid-wide barrier of the contact rebuild
+ * (default 30 s); a rebuild that gives up leaves PDGPU_ERR_CUDA on the context,
+ * from which pdgpu_load_state recovers.  0 gives up at the first poll. */
+PDGPU_API int pdgpu_set_barrier_limit(pdgpu_ctx *ctx, int64_t ns);
+
 /* A batched ensemble (no counterpart in the reference, which runs one scene
  * per process): the uploaded nodes and particles hold n_scenes independent
  * scenes, each a contiguous run of particles (particle_offsets, n_scenes + 1

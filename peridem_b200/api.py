@@ -111,6 +111,7 @@ SIGNATURES = {
     "pdgpu_write_strain_vtu": [c_vp, ctypes.c_char_p, c_i64, P(c_d), P(c_d), P(c_d)],
     "pdgpu_enable_rebuild_phases": [c_vp, c_i32],
     "pdgpu_rebuild_phases": [c_vp, P(c_i64), c_i32, P(c_i32)],
+    "pdgpu_set_barrier_limit": [c_vp, c_i64],
     "pdgpu_compute_pd_forces": [c_vp],
     "pdgpu_set_tile_nodes": [c_vp, c_i32],
     "pdgpu_tc_gemm": [c_vp, c_i32, c_vp, c_i32, c_i32, c_i32, c_i32, c_vp, c_i32, c_vp, c_vp, c_i32,

@@ -216,6 +216,7 @@ struct DevData {
   int32_t contact_grid;  // blocks of the contact node pass
   Grid grid;
   int32_t *cell_of, *cell_cnt, *cell_start, *cell_fill, *cell_tmp, *cell_nodes;
+  unsigned long long bar_wait_ns;  // longest wait at a barrier of the contact rebuild
   // contact rebuild, per node in cell order: its particle and position
   int32_t *cell_p;
   double *cell_x;

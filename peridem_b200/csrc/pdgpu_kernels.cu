@@ -602,20 +602,19 @@ constexpr int kCoopBlock = 256;
 // a counter in the step-control state; the last to arrive resets it and
 // advances the generation the others poll.  All blocks of the cooperative
 // launch are resident, so the wait ends unless a block faulted; after
-// kBarWaitNs of the GPU's global timer (far beyond any phase of a rebuild)
+// d.bar_wait_ns of the GPU's global timer (30 s by default, far beyond any phase)
 // the block records DEV_ERR_BARRIER_TIMEOUT and every block leaves the
 // rebuild at its next barrier (the step's later kernels see the error word
 // and do nothing).  Returns false when the rebuild must stop.
-constexpr unsigned long long kBarWaitNs = 30ull * 1000000000ull;
-
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
 
-__device__ bool grid_bar(CtrlState *c) {
+__device__ bool grid_bar(const DevData &d) {
   __shared__ int s_ok;
+  CtrlState *c = d.ctrl;
   __syncthreads();
   if (threadIdx.x == 0) {
     volatile unsigned *gen = &c->bar_gen;
@@ -627,12 +626,14 @@ __device__ bool grid_bar(CtrlState *c) {
       __threadfence();
       atomicAdd(&c->bar_gen, 1u);
     } else {
-      const unsigned long long t0 = global_ns();
+      const unsigned long long t0 = global_ns(), limit = d.bar_wait_ns;
+      const unsigned every = limit ? 255u : 0u;
       unsigned polls = 0;
       while (*gen == g0) {
-        // the clock is read every 256 polls; the poll count is a second,
-        // clock-independent bound (2^31 polls of at least a few ns each)
-        if ((++polls & 255u) == 0 && (global_ns() - t0 > kBarWaitNs || polls > (1u << 31))) {
+        // the clock is read every 256 polls (a limit of 0: at the first); the
+        // poll count is a second, clock-independent bound (2^31 polls of at
+        // least a few ns each)
+        if ((++polls & every) == 0 && (global_ns() - t0 >= limit || polls > (1u << 31))) {
           ok = 0;
           atomicCAS(&c->error, 0, DEV_ERR_BARRIER_TIMEOUT);
           break;
@@ -651,7 +652,7 @@ __device__ bool grid_bar(CtrlState *c) {
 // i = 0..n, each block scanning one contiguous chunk; false when a barrier
 // gave up
 template <class Tout, class F>
-__device__ bool grid_scan(CtrlState *gc, F in, Tout *out, int64_t n, int64_t *bsum) {
+__device__ bool grid_scan(const DevData &d, F in, Tout *out, int64_t n, int64_t *bsum) {
   __shared__ int64_t wsum[kCoopBlock / 32];
   __shared__ int64_t carry;
   const int64_t nb = gridDim.x;
@@ -669,7 +670,7 @@ __device__ bool grid_scan(CtrlState *gc, F in, Tout *out, int64_t n, int64_t *bs
     for (int w = 0; w < kCoopBlock / 32; w++) s += wsum[w];
     bsum[blockIdx.x] = s;
   }
-  if (!grid_bar(gc)) return false;
+  if (!grid_bar(d)) return false;
   {
     // carry = sum of the earlier blocks' totals, summed by the whole block
     // (integers: any order gives the same sum); read past L1, which may
@@ -708,7 +709,7 @@ __device__ bool grid_scan(CtrlState *gc, F in, Tout *out, int64_t n, int64_t *bs
     __syncthreads();
   }
   if (blockIdx.x == nb - 1 && threadIdx.x == 0) out[n] = (Tout)carry;
-  return grid_bar(gc);
+  return grid_bar(d);
 }
 
 
@@ -716,7 +717,7 @@ __device__ bool grid_scan(CtrlState *gc, F in, Tout *out, int64_t n, int64_t *bs
 // one pass over the nodes: emit(i, count, row start, compacted position); the
 // last block's totals go to tot[0], tot[1].  bsum: 2 values per block.
 template <class Emit>
-__device__ bool scan_rows(CtrlState *gc, const int64_t *cnt, int64_t n, int64_t *bsum, int64_t (&tot)[2], Emit emit) {
+__device__ bool scan_rows(const DevData &d, const int64_t *cnt, int64_t n, int64_t *bsum, int64_t (&tot)[2], Emit emit) {
   __shared__ int64_t wsum[2][kCoopBlock / 32];
   __shared__ int64_t carry[2];
   const int64_t nb = gridDim.x;
@@ -748,7 +749,7 @@ __device__ bool scan_rows(CtrlState *gc, const int64_t *cnt, int64_t n, int64_t 
     bsum[2 * blockIdx.x] = t[0];
     bsum[2 * blockIdx.x + 1] = t[1];
   }
-  if (!grid_bar(gc)) return false;
+  if (!grid_bar(d)) return false;
   // carry = sum of the earlier blocks' totals (integers: any order gives the
   // same sum), read past L1, which may hold this array from an earlier scan
   t[0] = t[1] = 0;
@@ -970,7 +971,6 @@ __global__ void __launch_bounds__(kCoopBlock, 4) k_contact_rebuild(const __grid_
     list_live_tiles(d);
     return;
   }
-  CtrlState *gc = d.ctrl;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   // phase clock (profiling): the first CTA's time past each barrier
   int mark = 0;
@@ -983,7 +983,8 @@ __global__ void __launch_bounds__(kCoopBlock, 4) k_contact_rebuild(const __grid_
   const int64_t nth = (int64_t)gridDim.x * blockDim.x;
   const int64_t N = d.n_nodes;
   const Grid G = d.grid;
-  // nodes per cell (the counters are zero between rebuilds)
+  // nodes per cell (the counters are zero between rebuilds; where a rebuild that
+  // stopped at a barrier is followed by others, the host clears them)
   if (d.sur_near_gate)
     for (int64_t p = tid; p < d.n_particles; p += nth) d.sur_near[p] = 0;
   for (int64_t i = tid; i < N; i += nth) {
@@ -993,16 +994,16 @@ __global__ void __launch_bounds__(kCoopBlock, 4) k_contact_rebuild(const __grid_
     d.cell_of[i] = c;
     atomicAdd(d.cell_cnt + c, 1);
   }
-  if (!grid_bar(gc)) return;
+  if (!grid_bar(d)) return;
   stamp();
   const int32_t *cc = d.cell_cnt;
-  if (!grid_scan<int32_t>(gc, [cc](int64_t k) { return cc[k]; }, d.cell_start, G.ncells, bsum)) return;
+  if (!grid_scan<int32_t>(d, [cc](int64_t k) { return cc[k]; }, d.cell_start, G.ncells, bsum)) return;
   stamp();
   for (int64_t i = tid; i < N; i += nth) {
     const int c = d.cell_of[i];
     d.cell_tmp[d.cell_start[c] + atomicAdd(d.cell_fill + c, 1)] = (int32_t)i;
   }
-  if (!grid_bar(gc)) return;
+  if (!grid_bar(d)) return;
   stamp();
   {
     // per cell: its nodes in index order (rank counting), their particles and
@@ -1036,14 +1037,14 @@ __global__ void __launch_bounds__(kCoopBlock, 4) k_contact_rebuild(const __grid_
       }
     }
   }
-  if (!grid_bar(gc)) return;
+  if (!grid_bar(d)) return;
   stamp();
   cand_count<DIM, DIM == 2 ? kCandLanes2 : kCandLanes3>(d, search_bit);
-  if (!grid_bar(gc)) return;
+  if (!grid_bar(d)) return;
   stamp();
   // row offsets and the compacted list of nodes with candidates
   int64_t tot[2];
-  const bool ok = scan_rows(gc, d.c_cnt, N, bsum, tot, [&](int64_t i, int64_t cnt, int64_t row, int64_t at) {
+  const bool ok = scan_rows(d, d.c_cnt, N, bsum, tot, [&](int64_t i, int64_t cnt, int64_t row, int64_t at) {
     d.c_row[i] = row;
     if (cnt > 0) {
       d.c_nodes[at] = (int32_t)i;
@@ -1056,7 +1057,7 @@ __global__ void __launch_bounds__(kCoopBlock, 4) k_contact_rebuild(const __grid_
     d.c_row[N] = tot[0];
     d.ctrl->c_nnodes = tot[1];
   }
-  if (!grid_bar(gc)) return;
+  if (!grid_bar(d)) return;
   list_live_tiles(d);  // the proximity flags are final
   for (int k = 0; k < 3; k++) stamp();  // row offsets, compaction offsets, lists: one pass
   cand_fill_nodes<DIM>(d, d.ctrl->c_nnodes);

@@ -1331,6 +1331,7 @@ int pdgpu_create(const pdgpu_desc *desc, pdgpu_ctx **out) {
   d.precision = desc->precision;
   d.dt = desc->dt;
   d.restart_step = -1;
+  d.bar_wait_ns = 30ull * 1000000000ull;
   for (int q = 0; q < 3; q++) d.gravity[q] = desc->gravity[q];
   const double gl = std::sqrt(desc->gravity[0] * desc->gravity[0] + desc->gravity[1] * desc->gravity[1] +
                               desc->gravity[2] * desc->gravity[2]);
@@ -2671,6 +2672,17 @@ int pdgpu_write_strain_vtu(pdgpu_ctx *ctx, const char *path, int64_t n_points, c
   return PDGPU_OK;
 }
 
+int pdgpu_set_barrier_limit(pdgpu_ctx *ctx, int64_t ns) {
+  if (!ctx) return PDGPU_ERR_ARG;
+  if (ns < 0) return fail(ctx, PDGPU_ERR_ARG, "set_barrier_limit: %lld ns", (long long)ns);
+  ctx->d.bar_wait_ns = (unsigned long long)ns;
+  if (ctx->gexec) {  // kernels in a graph hold the DevData they were captured with
+    cudaGraphExecDestroy(ctx->gexec);
+    ctx->gexec = nullptr;
+  }
+  return PDGPU_OK;
+}
+
 int pdgpu_enable_rebuild_phases(pdgpu_ctx *ctx, int32_t on) {
   if (!ctx) return PDGPU_ERR_ARG;
   DevData &d = ctx->d;
@@ -2978,6 +2990,10 @@ int pdgpu_load_state(pdgpu_ctx *ctx, const char *path) {
     CK(cudaGetLastError());
     TRY(ul(ctx, d.wp, wp));
     TRY(ul(ctx, d.wp_cnt, wpc));
+    // the error this clears may be of a rebuild that stopped with nodes counted
+    // in its cells: the next one counts from zero
+    CK(cudaMemsetAsync(d.cell_cnt, 0, ((size_t)d.grid.ncells + 1) * 4, ctx->stream));
+    CK(cudaMemsetAsync(d.cell_fill, 0, ((size_t)d.grid.ncells + 1) * 4, ctx->stream));
     CK(cudaMemsetAsync(d.fc, 0, (size_t)(st * N) * 8, ctx->stream));
   }
   TRY(ul(ctx, d.history, hist));
