@@ -530,7 +530,7 @@ bool limit_law(size_t bytes) {
       (const void *)k_bonds_fp64<DIM, 16, LAW, PRE, uint16_t>, (const void *)k_bonds_fp64<DIM, 32, LAW, PRE, uint16_t>,
       (const void *)k_bonds_fp64<DIM, 8, LAW, PRE, int32_t>,   (const void *)k_bonds_fp64<DIM, 8, LAW, PRE, void>};
   for (auto f : fs)
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) return false;
+    if (!allow_smem(f, bytes)) return false;
   return true;
 }
 

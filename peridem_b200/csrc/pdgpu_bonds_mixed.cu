@@ -782,8 +782,7 @@ bool set_law_limit(size_t bytes) {
                       (const void *)k_bonds_mixed<DIM, 16, LAW, CT, PRE, SYM>,
                       (const void *)k_bonds_mixed<DIM, 32, LAW, CT, PRE, SYM>};
   for (auto f : fs)
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess)
-      return false;
+    if (!allow_smem(f, bytes)) return false;
   return true;
 }
 

@@ -438,6 +438,10 @@ void launch_prepass_mixed(const DevData &d, const BondTile *tiles, const int *la
                           size_t smem, cudaStream_t s);
 size_t tile_smem_fp64(int dim, bool state, int stage, bool col16, const BondTile &t);
 size_t tile_smem_mixed_main(int dim, bool state, bool col16, const BondTile &t, bool sym = false);
+// lets a kernel take `bytes` of dynamic shared memory.  The limit belongs to the
+// device's context, so every model of the process shares it: it only rises, and
+// a model whose tiles need more than a later one's keeps launching
+bool allow_smem(const void *kernel, size_t bytes);
 int set_tile_smem_limit_fp64(int dim, size_t bytes);
 int set_tile_smem_limit_mixed(int dim, size_t bytes);
 

@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -1278,6 +1279,15 @@ int build_graph(pdgpu_ctx *ctx, int steps) {
 }
 
 }  // namespace
+
+bool pdgpu::allow_smem(const void *kernel, size_t bytes) {
+  static std::mutex one_at_a_time;  // two models may be preparing
+  std::lock_guard<std::mutex> lock(one_at_a_time);
+  cudaFuncAttributes a;
+  if (cudaFuncGetAttributes(&a, kernel) != cudaSuccess) return false;
+  return (size_t)a.maxDynamicSharedSizeBytes >= bytes ||
+         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) == cudaSuccess;
+}
 
 // ===========================================================================
 // C ABI
