@@ -84,6 +84,12 @@ __device__ __forceinline__ double quot(double a, double b, double y) {
   return __fma_rn(__fma_rn(-b, q, a), y, q);
 }
 
+// the same where the quotient may be infinite (its residual is not a number then)
+__device__ __forceinline__ double quot_or_inf(double a, double b, double y) {
+  const double q = a * y, c = __fma_rn(__fma_rn(-b, q, a), y, q);
+  return c == c ? c : q;
+}
+
 // Shared-memory plan of one tile (byte offsets), identical on host and
 // device.  The window's node data always sit in shared memory; where it is
 // too wide for the rest, first the state law's {3K/m - 5G/m, 15G/m} pairs, then
@@ -213,7 +219,9 @@ struct Sum64 {
 // a bond that breaks carries no force and repels from the next evaluation on.
 // Without TEST neither is looked at: a node none of whose bonds starts broken
 // is summed that way first, and again with TEST only when its largest stretch
-// measure could break a bond (the caller's decision).  RANGE: every reference
+// measure could break a bond or a stretch may have overflowed (the caller's
+// decision): only TEST yields an infinite stretch, where the other yields NaN,
+// which the largest measure passes over.  RANGE: every reference
 // distance of the lists is inside root_in_range's.
 template <int DIM, int LAW, bool PRE, bool TEST, bool RANGE>
 __device__ __forceinline__ bool bond64(const Bond64<DIM> &B, const Node64 &I, int lj, bool broken, Sum64 &s) {
@@ -232,10 +240,11 @@ __device__ __forceinline__ bool bond64(const Bond64<DIM> &B, const Node64 &I, in
   const double r2 = dotd<DIM>(dx, dx);
   const Root R = RANGE ? root_in_range(r2) : root(r2);
   const double rji = R.r;
+  auto stretch = [](double a, double b, double y) { return TEST ? quot_or_inf(a, b, y) : quot(a, b, y); };
   bool breaks = false;
   double S, ly = 0.0, inv_ly = 0.0, cl = 0.0;
   if constexpr (LAW == LAW_RNP) {
-    S = quot(dotd<DIM>(dx, du), r2, R.inv * R.inv);
+    S = stretch(dotd<DIM>(dx, du), r2, R.inv * R.inv);
     const double zq = S * S * rji;  // Z = |S| sqrt(r) / rbar
     s.zmax = zq > s.zmax ? zq : s.zmax;
   } else {
@@ -243,7 +252,7 @@ __device__ __forceinline__ bool bond64(const Bond64<DIM> &B, const Node64 &I, in
     ly = L.r;
     inv_ly = L.inv;
     cl = ly - rji;
-    S = quot(cl, rji, R.inv);
+    S = stretch(cl, rji, R.inv);
     const double za = fabs(S);
     s.zmax = za > s.zmax ? za : s.zmax;
   }
@@ -425,6 +434,8 @@ __global__ void __launch_bounds__(kThreads64<DIM>, DIM == 2 ? 4 : 1)
     }
     s.zmax = gmax64<LPN>(s.zmax);
     test |= may_break && !(s.zmax <= break_z);
+    // a stretch that overflowed leaves its lane's force not a number
+    if constexpr (!PRE) test |= !(fabs(s.f[0]) + fabs(s.f[1]) + fabs(s.f[2]) <= DBL_MAX);
     if (__any_sync(kFullWarp, test)) {
       if (test) {
         s = Sum64{};
