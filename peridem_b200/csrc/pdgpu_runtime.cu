@@ -528,7 +528,6 @@ int prepare_fp64(pdgpu_ctx *ctx) {
   bool state = false;
   for (const auto &P : ctx->hp) state |= P.material == PDGPU_MAT_PDSTATE && P.compute_force;
   if (state) TRY(dalloc(ctx, &d.fa, d.n_nodes));
-  d.inf_inv_p1 = 1.0 / d.inf.p1;
   TRY(alloc_col16(ctx));
   launch_mixed_setup(d, ctx->stream);
   int32_t *out;
@@ -1513,6 +1512,7 @@ int pdgpu_set_influence(pdgpu_ctx *ctx, int32_t type, const double params[2]) {
   ctx->d.inf.type = type;
   ctx->d.inf.p0 = params[0];
   ctx->d.inf.p1 = params[1];
+  ctx->d.inf_inv_p1 = 1.0 / params[1];  // the FP64 form takes both from here, at any time
   return PDGPU_OK;
 }
 
