@@ -197,9 +197,9 @@ struct Bond64 {
 };
 
 template <int LPN>
-__device__ __forceinline__ double gmax64(double v) {
+__device__ __forceinline__ double gmax64(double v, int lanes) {
 #pragma unroll
-  for (int o = LPN / 2; o > 0; o >>= 1) {
+  for (int o = (LPN ? LPN : lanes) / 2; o > 0; o >>= 1) {
     const double b = __shfl_xor_sync(kFullWarp, v, o);
     v = b > v ? b : v;
   }
@@ -307,10 +307,11 @@ __device__ __forceinline__ bool bond64(const Bond64<DIM> &B, const Node64 &I, in
 // particle-local or int32_t global); COL = void reads whatever form the
 // columns have, with the row offsets and bitmap, from global memory (tiles
 // whose window leaves no room, and reference distances outside the range of
-// the unchecked root).
+// the unchecked root).  LPN lanes per node; LPN = 0, of the last two, whose
+// scenes are rare: as many as `lanes` says.
 template <int DIM, int LPN, int LAW, bool PRE, typename COL>
 __global__ void __launch_bounds__(kThreads64<DIM>, DIM == 2 ? 4 : 1)
-    k_bonds_fp64(const __grid_constant__ DevData d, const BondTile *__restrict__ tiles, int stage) {
+    k_bonds_fp64(const __grid_constant__ DevData d, const BondTile *__restrict__ tiles, int stage, int lanes) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ __align__(8) uint64_t bar;
   constexpr int kT = kThreads64<DIM>;
@@ -387,7 +388,7 @@ __global__ void __launch_bounds__(kThreads64<DIM>, DIM == 2 ? 4 : 1)
 
   B.V = Win<DIM>{reinterpret_cast<const double2 *>(smem + p.off_x), s_u, s_z,
                  reinterpret_cast<const double *>(smem + p.off_vol) + (T.win_begin - p.vol0)};
-  const int lane = threadIdx.x % LPN;
+  const int lpn = LPN ? LPN : lanes, lane = threadIdx.x & (lpn - 1);
   const int64_t kb = T.bond_begin;
   // bond indices are relative to the tile's first bond; the bitmap's to the
   // word that holds it
@@ -409,10 +410,10 @@ __global__ void __launch_bounds__(kThreads64<DIM>, DIM == 2 ? 4 : 1)
   // (RNP) or |S| is at most break_z
   const bool may_break = LAW == LAW_RNP ? B.irrev : (LAW == LAW_PMB || PRE);
   const double break_z = LAW == LAW_RNP ? P.break_q : (LAW == LAW_PMB ? B.m1 : B.m2);
-  // a warp's 32 / LPN nodes go through the loop together; past the tile's end
+  // a warp's 32 / lpn nodes go through the loop together; past the tile's end
   // a group has an empty row
-  for (int64_t wb = T.node_begin + threadIdx.x / 32 * (32 / LPN); wb < T.node_end; wb += kT / LPN) {
-    const int64_t i_raw = wb + (threadIdx.x & 31) / LPN;
+  for (int64_t wb = T.node_begin + threadIdx.x / 32 * (32 / lpn); wb < T.node_end; wb += kT / lpn) {
+    const int64_t i_raw = wb + (threadIdx.x & 31) / lpn;
     const bool in_tile = i_raw < T.node_end;
     const int64_t i = in_tile ? i_raw : T.node_end - 1;
     const int li = (int)(i - T.win_begin);
@@ -427,12 +428,12 @@ __global__ void __launch_bounds__(kThreads64<DIM>, DIM == 2 ? 4 : 1)
       I.a = q.y;
     }
     Sum64 s{};
-    bool test = any_broken<LPN>(bits, k0 + bit_off, k1 + bit_off);
+    bool test = any_broken<LPN>(bits, k0 + bit_off, k1 + bit_off, lpn);
     if (!test) {
 #pragma unroll 1
-      for (int k = k0 + lane; k < k1; k += LPN) bond64<DIM, LAW, PRE, false, kStaged>(B, I, neighbour(k), false, s);
+      for (int k = k0 + lane; k < k1; k += lpn) bond64<DIM, LAW, PRE, false, kStaged>(B, I, neighbour(k), false, s);
     }
-    s.zmax = gmax64<LPN>(s.zmax);
+    s.zmax = gmax64<LPN>(s.zmax, lpn);
     test |= may_break && !(s.zmax <= break_z);
     // a stretch that overflowed leaves its lane's force not a number
     if constexpr (!PRE) test |= !(fabs(s.f[0]) + fabs(s.f[1]) + fabs(s.f[2]) <= DBL_MAX);
@@ -440,21 +441,21 @@ __global__ void __launch_bounds__(kThreads64<DIM>, DIM == 2 ? 4 : 1)
       if (test) {
         s = Sum64{};
 #pragma unroll 1
-        for (int k = k0 + lane; k < k1; k += LPN) {
+        for (int k = k0 + lane; k < k1; k += lpn) {
           const int b = k + bit_off;
           const bool broken = (bits[b >> 5] >> (b & 31)) & 1u;
           if (bond64<DIM, LAW, PRE, true, kStaged>(B, I, neighbour(k), broken, s)) break_bond(k);
         }
       }
       __syncwarp();
-      s.zmax = gmax64<LPN>(s.zmax);
+      s.zmax = gmax64<LPN>(s.zmax, lpn);
     }
     if constexpr (PRE) {
-      s.theta = gsum<LPN>(s.theta);
+      s.theta = gsum<LPN>(s.theta, lpn);
       if (lane == 0 && in_tile) d.theta[i] = 3.0 * s.theta / d.mx[i];
     } else {
 #pragma unroll
-      for (int q = 0; q < DIM; q++) s.f[q] = gsum<LPN>(s.f[q]);
+      for (int q = 0; q < DIM; q++) s.f[q] = gsum<LPN>(s.f[q], lpn);
       if (lane == 0 && in_tile) {
         reinterpret_cast<double2 *>(d.f)[DIM == 2 ? i : 2 * i] = make_double2(s.f[0], s.f[1]);
         if constexpr (DIM == 3) d.f[4 * i + 2] = s.f[2];
@@ -502,20 +503,20 @@ __global__ void k_fp64_range(const __grid_constant__ DevData d, int32_t *outside
 }
 
 template <int DIM, int LPN, int LAW, bool PRE, typename COL>
-void launch_one(const DevData &d, const BondTile *t, int n, int stage, size_t smem, cudaStream_t s) {
+void launch_one(const DevData &d, const BondTile *t, int n, int lanes, int stage, size_t smem, cudaStream_t s) {
   // behind the pre-pass (see launch_one of the FP32 form for the others)
-  if constexpr (LAW == LAW_STATE && !PRE) launch_dependent(k_bonds_fp64<DIM, LPN, LAW, PRE, COL>, n, kThreads64<DIM>, smem, s, d, t, stage);
-  else k_bonds_fp64<DIM, LPN, LAW, PRE, COL><<<n, kThreads64<DIM>, smem, s>>>(d, t, stage);
+  if constexpr (LAW == LAW_STATE && !PRE) launch_dependent(k_bonds_fp64<DIM, LPN, LAW, PRE, COL>, n, kThreads64<DIM>, smem, s, d, t, stage, lanes);
+  else k_bonds_fp64<DIM, LPN, LAW, PRE, COL><<<n, kThreads64<DIM>, smem, s>>>(d, t, stage, lanes);
 }
 
 template <int DIM, int LAW, bool PRE>
 void launch_lanes(const DevData &d, const BondTile *t, int n, int lanes, int stage, size_t smem, cudaStream_t s) {
-  if (!(stage & ST_BONDS)) launch_one<DIM, 8, LAW, PRE, void>(d, t, n, stage, smem, s);
-  else if (!d.use16) launch_one<DIM, 8, LAW, PRE, int32_t>(d, t, n, stage, smem, s);
-  else if (lanes == 4) launch_one<DIM, 4, LAW, PRE, uint16_t>(d, t, n, stage, smem, s);
-  else if (lanes == 8) launch_one<DIM, 8, LAW, PRE, uint16_t>(d, t, n, stage, smem, s);
-  else if (lanes == 16) launch_one<DIM, 16, LAW, PRE, uint16_t>(d, t, n, stage, smem, s);
-  else launch_one<DIM, 32, LAW, PRE, uint16_t>(d, t, n, stage, smem, s);
+  if (!(stage & ST_BONDS)) launch_one<DIM, 0, LAW, PRE, void>(d, t, n, lanes, stage, smem, s);
+  else if (!d.use16) launch_one<DIM, 0, LAW, PRE, int32_t>(d, t, n, lanes, stage, smem, s);
+  else if (lanes == 4) launch_one<DIM, 4, LAW, PRE, uint16_t>(d, t, n, lanes, stage, smem, s);
+  else if (lanes == 8) launch_one<DIM, 8, LAW, PRE, uint16_t>(d, t, n, lanes, stage, smem, s);
+  else if (lanes == 16) launch_one<DIM, 16, LAW, PRE, uint16_t>(d, t, n, lanes, stage, smem, s);
+  else launch_one<DIM, 32, LAW, PRE, uint16_t>(d, t, n, lanes, stage, smem, s);
 }
 
 template <int DIM>
@@ -539,7 +540,7 @@ bool limit_law(size_t bytes) {
   const void *fs[] = {
       (const void *)k_bonds_fp64<DIM, 4, LAW, PRE, uint16_t>,  (const void *)k_bonds_fp64<DIM, 8, LAW, PRE, uint16_t>,
       (const void *)k_bonds_fp64<DIM, 16, LAW, PRE, uint16_t>, (const void *)k_bonds_fp64<DIM, 32, LAW, PRE, uint16_t>,
-      (const void *)k_bonds_fp64<DIM, 8, LAW, PRE, int32_t>,   (const void *)k_bonds_fp64<DIM, 8, LAW, PRE, void>};
+      (const void *)k_bonds_fp64<DIM, 0, LAW, PRE, int32_t>,   (const void *)k_bonds_fp64<DIM, 0, LAW, PRE, void>};
   for (auto f : fs)
     if (!allow_smem(f, bytes)) return false;
   return true;

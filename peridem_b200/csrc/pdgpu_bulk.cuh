@@ -57,12 +57,13 @@ __device__ __forceinline__ bool bar_wait(uint64_t *bar, uint32_t parity) {
 // after the other from there on (FP64 bond loop at 8 lanes per node, 2-D
 // compression of 333 000 nodes: 363 us with a mask per group, 169 us with one;
 // FP32 form in 3-D, pre-pass 100 and 85 us).
+// LPN = 0: `lanes` of them, a power of two up to 32, known at run time.
 constexpr unsigned kFullWarp = 0xffffffffu;
 
 template <int LPN>
-__device__ __forceinline__ double gsum(double v) {
+__device__ __forceinline__ double gsum(double v, int lanes = LPN) {
 #pragma unroll
-  for (int o = LPN / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFullWarp, v, o);
+  for (int o = (LPN ? LPN : lanes) / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFullWarp, v, o);
   return v;
 }
 template <int LPN>
@@ -74,12 +75,12 @@ __device__ __forceinline__ float gmax(float v) {
 
 // does any bond of [b0, b1) (bit positions in a bitmap) start broken?
 template <int LPN>
-__device__ __forceinline__ bool any_broken(const uint32_t *bits, int b0, int b1) {
-  const int lane = threadIdx.x % LPN;
+__device__ __forceinline__ bool any_broken(const uint32_t *bits, int b0, int b1, int lanes = LPN) {
+  const int lpn = LPN ? LPN : lanes, lane = threadIdx.x & (lpn - 1);
   const int w0 = b0 >> 5, w1 = (b1 - 1) >> 5;
   bool hit = false;
   if (b1 > b0)
-    for (int w = w0 + lane; w <= w1; w += LPN) {
+    for (int w = w0 + lane; w <= w1; w += lpn) {
       uint32_t m = bits[w];
       if (w == w0) m &= ~0u << (b0 & 31);
       if (w == w1) m &= ~0u >> (31 - ((b1 - 1) & 31));
@@ -87,8 +88,8 @@ __device__ __forceinline__ bool any_broken(const uint32_t *bits, int b0, int b1)
     }
   if constexpr (LPN == 1) return hit;
   const unsigned all = __ballot_sync(kFullWarp, hit);
-  if constexpr (LPN == 32) return all != 0u;
-  return (all >> ((threadIdx.x & 31u) / LPN * LPN)) & ((1u << (LPN & 31)) - 1u);
+  // the group's lanes of the 32
+  return ((all >> (threadIdx.x & 31u & ~(lpn - 1u))) & (kFullWarp >> (32 - lpn))) != 0u;
 }
 
 }  // namespace
