@@ -40,7 +40,7 @@ def _nvcc():
 
 def sources():
     return [os.path.join(CSRC, u) for u, _ in UNITS] + [
-        *(os.path.join(CSRC, h) for h in ("pdgpu_internal.h", "pdgpu_bulk.cuh", "pdgpu_pdl.cuh")),
+        *(os.path.join(CSRC, h) for h in ("pdgpu_internal.h", "pdgpu_bulk.cuh", "pdgpu_pdl.cuh", "pdgpu_quot.cuh")),
         os.path.join(ROOT, "include", "pdgpu.h")]
 
 

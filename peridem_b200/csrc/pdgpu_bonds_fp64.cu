@@ -1,7 +1,7 @@
 // Tiled bond loop of DEMModel::computePeridynamicForces
 // (demModel.cpp:602-789), FP64 form: the reference's arithmetic (compiled with
-// --fmad=false; its order of operations, every quotient and square root
-// rounded once).
+// --fmad=false; its order of operations, quotients and square roots rounded to
+// nearest but for the cases pdgpu_quot.cuh names).
 //
 // One CTA per tile of one particle's nodes.  The tile's neighbour columns,
 // row offsets and words of the broken-bond bitmap and the window of nodes its
@@ -9,18 +9,12 @@
 // only shared memory; each law is its own instantiation.
 //
 // What bounds it: the FP64 pipe (64 lanes per SM) and the latency of its
-// chains.  The compiler's FP64 divide and square root cost 10-20 instructions
-// each, and a bond needs up to 13 of them; here
-//   * sqrt(a) and 1/sqrt(a) come together from the hardware approximation and
-//     one third-order step (Householder), the root then corrected by its exact
-//     residual (Markstein);
-//   * a quotient a/b is a y corrected once by its exact residual, y ~ 1/b
-//     being at hand (Markstein, "Computation of elementary functions on the
-//     IBM RISC System/6000 processor", 1990): the correctly rounded value, as
-//     the divide instruction sequence gives it, at three operations;
+// chains.  A bond needs up to 13 quotients and roots, many instructions each as
+// plain divisions and sqrt; here
+//   * sqrt(a), 1/sqrt(a) and quotients by one correction each (pdgpu_quot.cuh),
+//     a quotient at three operations;
 //   * quantities of one node (15 G / m_x, 3 K / m_x - 5 G / m_x) are computed
 //     once per node at set-up instead of once per bond.
-// Roots outside [2^-900, 2^892] take the compiler's sqrt and divide.
 // A node is summed without tests of broken or breaking bonds first; the tests
 // run in a second sum of that node where they can matter.
 //
@@ -41,6 +35,7 @@
 #include "pdgpu_bulk.cuh"
 #include "pdgpu_internal.h"
 #include "pdgpu_pdl.cuh"
+#include "pdgpu_quot.cuh"
 
 namespace pdgpu {
 namespace {
@@ -56,38 +51,6 @@ enum { LAW_RNP = 0, LAW_PMB = 1, LAW_ELASTIC = 2, LAW_STATE = 3 };
 __device__ __forceinline__ bool gt(double a, double b) {
   const double fa = fabs(a), fb = fabs(b);
   return (a - b) > ((fa < fb ? fb : fa) * 1.0e-5);
-}
-
-struct Root {
-  double r, inv;  // sqrt(a) correctly rounded, 1/sqrt(a) to about one ulp
-};
-
-// a inside [2^-900, 2^892]
-__device__ __forceinline__ Root root_in_range(double a) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
-  // 1/sqrt(a) = y (1 - e)^(-1/2) with e = 1 - a y^2, to second order in e
-  const double e = __fma_rn(-(a * y), y, 1.0);
-  y = __fma_rn(y * e, __fma_rn(e, 0.375, 0.5), y);
-  const double r0 = a * y;
-  return Root{__fma_rn(__fma_rn(-r0, r0, a), 0.5 * y, r0), y};
-}
-__device__ __forceinline__ Root root(double a) {
-  if ((unsigned)(__double2hiint(a) - 0x07b00000) < 0x70000000u) return root_in_range(a);
-  const double r = sqrt(a);
-  return Root{r, 1.0 / r};
-}
-
-// a / b, given y ~ 1/b
-__device__ __forceinline__ double quot(double a, double b, double y) {
-  const double q = a * y;
-  return __fma_rn(__fma_rn(-b, q, a), y, q);
-}
-
-// the same where the quotient may be infinite (its residual is not a number then)
-__device__ __forceinline__ double quot_or_inf(double a, double b, double y) {
-  const double q = a * y, c = __fma_rn(__fma_rn(-b, q, a), y, q);
-  return c == c ? c : q;
 }
 
 // Shared-memory plan of one tile (byte offsets), identical on host and
