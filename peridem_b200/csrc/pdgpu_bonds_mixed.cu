@@ -695,10 +695,13 @@ __global__ void __launch_bounds__(kThreadsFor<DIM, LPN>) k_bonds_mixed(DevData d
 }
 
 // CTAs per SM for the persistent bond loop: the occupancy limit (the contact
-// pass is placed ahead of it); with the learned surrogate, whose chain runs on a
-// third stream beside it, one less where at least three fit.  (One slot left
-// free for all: 332 000 nodes 49.3 us a step against 48.5, 1.3 M nodes 160.8
-// against 154.2.)
+// pass is placed ahead of it; one slot left free for all: 332 000 nodes 49.3 us a
+// step against 48.5, 1.3 M nodes 160.8 against 154.2).  With the learned
+// surrogate, whose chain runs on a third stream beside it, the chain's CTAs of
+// 256 and 512 threads need more than one slot of 128: of ten slots three stay
+// free (2 000 bodies, 1.3 M nodes, 81 % of them on the surrogate, us a step with
+// 0 / 1 / 2 / 3 / 4 free: 124.1 / 124.3 / 124.6 / 121.2 / 122.6; 502 bodies, 72 %:
+// 43.3 / 43.3 / - / 43.4), of three or four one.
 template <class K>
 int bond_grid(K kernel, int threads, size_t smem, int n_tiles, bool surrogate) {
   static int sms = 0;
@@ -710,7 +713,8 @@ int bond_grid(K kernel, int threads, size_t smem, int n_tiles, bool surrogate) {
   }
   int per = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, threads, smem);
-  const int g = sms * (surrogate && per > 2 ? per - 1 : (per > 0 ? per : 1));
+  const int keep = !surrogate ? 0 : per > 4 ? 3 : per > 2 ? 1 : 0;
+  const int g = sms * (per > 0 ? per - keep : 1);
   return g < n_tiles ? g : n_tiles;
 }
 
