@@ -406,8 +406,8 @@ PDGPU_API int pdgpu_download_pd_neighbors(pdgpu_ctx *ctx, uint64_t *rowptr, uint
  * per node.  0 keeps the current choice.  Set before the first step. */
 PDGPU_API int pdgpu_set_tuning(pdgpu_ctx *ctx, int32_t pd_lanes, int32_t contact_lanes);
 
-/* CTAs per SM of the contact node pass (1..16, by default 1 or 2 by the
- * scene's size); it runs beside
+/* CTAs per SM of the contact node pass (1..16; by default 1 or 2 by the
+ * scene's size, 2 with more than one contact lane per node); it runs beside
  * the bond loop and is bound by the latency of its gathers.  Set before the
  * first step. */
 PDGPU_API int pdgpu_set_contact_grid(pdgpu_ctx *ctx, int32_t ctas_per_sm);

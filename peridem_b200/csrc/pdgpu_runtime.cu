@@ -928,13 +928,19 @@ int prepare(pdgpu_ctx *ctx) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    // Two CTAs per SM, one in scenes of medium size: the bond loop's first
-    // CTAs wait for the contact pass's, so where one CTA per SM gets through
-    // the candidates quickly the bond loop starts earlier (us per step with one
-    // / two: 332 000 nodes FP32 form 48.0 / 49.4, FP64 90.0 / 91.8, an ensemble
-    // of 416 000 55.1 / 56.0; but 24 000 nodes 25.0 / 23.7, where the pass is
-    // the longest chain beside a short bond loop, and 1.3 M 155.9 / 154.3)
-    if (ctx->contact_ctas <= 0) ctx->contact_ctas = N > kTurnMaxNodes && N <= 4 * kTurnMaxNodes ? 1 : 2;
+    // One contact lane per node: two CTAs per SM, one in scenes of medium size.
+    // The bond loop's first CTAs wait for the contact pass's, so where one CTA
+    // per SM gets through the candidates quickly the bond loop starts earlier
+    // (us per step with one / two: FP32 form, 2-D, 165 000 nodes 34.3 / 34.0,
+    // 252 000 40.7 / 43.9, 332 000 48.0 / 49.4, 590 000 75.7 / 77.3; FP64, 165 000
+    // 54.1 / 55.8, 590 000 151.7 / 153.7; 3-D, 168 000 106.9 / 107.9, 494 000
+    // 279.7 / 280.8; an ensemble of 416 000 55.1 / 56.0; but 24 000 nodes 25.0 /
+    // 23.7, where the pass is the longest chain beside a short bond loop, and
+    // 1.3 M 155.9 / 154.3.  The range is narrower than where one is the better:
+    // 125 000 nodes 28.0 / 29.1, 849 000 104.7 / 106.3).  More lanes per node
+    // want both (165 000 nodes, four lanes 53.8 / 42.1, 32 lanes 48.5 / 40.3).
+    if (ctx->contact_ctas <= 0)
+      ctx->contact_ctas = ctx->contact_lanes == 1 && N > kTurnMaxNodes && N <= 4 * kTurnMaxNodes ? 1 : 2;
     d.contact_grid = ctx->contact_ctas * (sms > 0 ? sms : 148);
   }
   d.cr_blocks = d.contact_grid;
