@@ -40,12 +40,14 @@ namespace mixed_loop {
 
 // threads per CTA: 128 in 2-D (fewer warps to wait for one another at a
 // tile's barriers, and the last tile of a particle wastes less than with 256:
-// 332 000 nodes 28.5 us against 30.5, 1.3 M nodes 77 against 84); in 3-D, where
-// a tile's neighbour window is large (~100 KB of stage) and only two CTAs fit
-// an SM, up to 512, so that two CTAs per SM (one computing while the other
-// waits at a tile barrier) fit the register file
+// 332 000 nodes 28.5 us against 30.5, 1.3 M nodes 77 against 84), 256 from 16
+// lanes per node on, where 128 threads would be eight nodes or fewer at a time
+// (24 000 nodes in tiles of 128, us a step with 128 / 256 threads: 16 lanes
+// 40.0 / 29.2, 32 lanes 59.5 / 41.0); in 3-D, where a tile's neighbour window is large
+// (~100 KB of stage) and only two CTAs fit an SM, up to 512, so that two CTAs per
+// SM (one computing while the other waits at a tile barrier) fit the register file
 template <int DIM, int LPN>
-constexpr int kThreadsFor = DIM == 3 ? (256 * LPN < 512 ? 256 * LPN : 512) : 128;
+constexpr int kThreadsFor = DIM == 3 ? (256 * LPN < 512 ? 256 * LPN : 512) : (LPN < 16 ? 128 : 256);
 
 // Shared-memory plan of one tile (byte offsets into the dynamic stage);
 // identical on host and device.  Bulk-copied regions start and end on 16-byte

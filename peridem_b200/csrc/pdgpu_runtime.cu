@@ -693,9 +693,13 @@ void choose_tiling(pdgpu_ctx *ctx) {
     if (mixed && d.dim == 3 && lanes0 == 1) ctx->tile_nodes = 256;  // one lane: 256 threads
     if (!mixed && d.dim == 2 && active > room * ctx->tile_nodes) ctx->tile_nodes *= 2;
   }
-  // every thread of the CTA has a node, and at least 128 (2-D) or 96 (3-D)
-  // nodes per tile
-  if (ctx->tile_nodes <= 0) ctx->tile_nodes = std::max<int64_t>(d.dim == 2 ? 128 : 96, 256 / ctx->pd_lanes);
+  // Lanes given, tile not: a node for every thread of the CTA, and at least 128
+  // nodes (2-D) or 96 (3-D) per tile; 2-D FP32 form, whose CTAs are smaller, 64
+  // (24 000 nodes, us a step with 128 / 64: 2 lanes 23.9 / 21.5, 8 lanes 35.0 / 27.9)
+  if (ctx->tile_nodes <= 0) {
+    const int64_t least = d.dim == 3 ? 96 : (mixed ? 64 : 128);
+    ctx->tile_nodes = std::max<int64_t>(least, (d.dim == 2 && mixed ? 128 : 256) / ctx->pd_lanes);
+  }
 }
 
 // Tiles of the bond loop: every force-computing particle is cut into runs of
