@@ -399,11 +399,16 @@ PDGPU_API int pdgpu_download_pd_neighbors(pdgpu_ctx *ctx, uint64_t *rowptr, uint
 /* Launch shape of the bond loop and the contact kernel: lanes per node
  * (4, 8, 16 or 32 for the bond loop, also 1 or 2 in the mixed form; 1, 2,
  * 4, 8 or 32 for the contact pass, default 1).  With 1 the contact pass is
- * one warp-cooperative kernel: a warp walks the candidate entries of 32
- * nodes, coalesced, and each node's lane adds its contributions in list
+ * one warp-cooperative kernel: a warp walks the candidate entries of 8, 16 or
+ * 32 nodes, coalesced, and each node's lane adds its contributions in list
  * order; with more, a flat distance pass marks the entries inside the
  * largest contact radius and a node pass sums them with that many lanes
- * per node.  0 keeps the current choice.  Set before the first step. */
+ * per node.  0 keeps the current choice.  Set before the first step.
+ * Lanes per node of the bond loop set the order in which a node's bonds are
+ * summed.  Without a choice here the FP64 form takes 4, 8 or 16 by the size of
+ * the whole scene and the GPU's SM count, so a body's forces may differ in
+ * their last bits between a scene alone and the same scene in an ensemble, or
+ * between GPUs with other SM counts; with pd_lanes set they do not. */
 PDGPU_API int pdgpu_set_tuning(pdgpu_ctx *ctx, int32_t pd_lanes, int32_t contact_lanes);
 
 /* CTAs per SM of the contact node pass (1..16; by default 1 or 2 by the

@@ -20,14 +20,19 @@
 //
 // Measured per launch (B200, us), against one CTA per tile with the compiler's
 // divides, the law chosen per bond and every operand in its own array:
-//   2-D, RNP, 333 000 nodes, 7.2 M bonds: 226 -> 74 (FP64 pipe 56 % busy, 82
-//   FP64 and 83 other thread instructions per bond; 40 us of FP64 issue);
-//   3-D, PD state, 75 000 sphere nodes, 6.5 M bonds: pre-pass 126 -> 54, main
-//   loop 337 -> 69; 3-D, PD elastic, 64 000 sphere nodes: 304 -> 55.
+//   2-D, RNP, 333 000 nodes, 7.6 M bonds: 226 -> 74 (FP64 pipe 59 % and issue
+//   71 % busy; 78 FP64 and 105 other thread instructions per bond, the nodes'
+//   own included);
+//   3-D, PD state, 75 000 sphere nodes, 6.4 M bonds: pre-pass 126 -> 54, main
+//   loop 337 -> 69 (FP64 pipe 48 and 53 %, issue 45 and 46 % at one CTA per SM);
+//   3-D, PD elastic, 63 000 sphere nodes, 5.3 M bonds: 304 -> 55 (54 %, 48 %).
 // The outputs are the same to the bit at equal lanes per node.  Four CTAs of
-// 256 threads per SM in 2-D (64 registers, 30 to 60 bytes of spills): a step of
-// the 333 000-node compression takes 91.8 us, with three (80 registers) 94.5;
-// with two (114 registers) the launch alone took a third longer.
+// 256 threads per SM in 2-D (64 registers; 32 to 84 bytes of spill stores and 36
+// to 116 of spill loads in the main loops): a step of the 333 000-node RNP
+// compression takes 91.8 us, with three (80 registers) 94.5; with two (114
+// registers) the launch alone took a third longer.  The other laws run that way
+// too; 151 000 nodes, us per step before and now: PMB 106.9 -> 45.8, PD elastic
+// 124.6 -> 47.7, PD state 173.8 -> 80.1.
 #include <cfloat>
 #include <cstdint>
 #include <type_traits>

@@ -20,13 +20,13 @@
 // comparisons util::isGreater (a - b > 1e-5 max(|a|, |b|)) become
 // comparisons against thresholds precomputed per particle.
 //
-// What bounds it: instruction issue (about 31 FP32 and 20 other thread
+// What bounds it: instruction issue (about 29 FP32 and 23 other thread
 // instructions per bond in 2-D, 57-65 % issue active) and, around it, the
 // barriers and loads at the start of each tile.  Measured per launch against
 // the loop with its break and influence tests inside, 256 threads per CTA and
 // every window node converted by its tile (B200, us, results the same to the
-// bit): 2-D RNP, 321 000 nodes, 7.2 M bonds 39 -> 26 beside the contact pass,
-// 1.26 M nodes 109 -> 82; 3-D PD state, 200 000 sphere nodes, 17.3 M bonds:
+// bit): 2-D RNP, 321 000 nodes, 7.6 M bonds 39 -> 26 beside the contact pass,
+// 1.26 M nodes 109 -> 82; 3-D PD state, 200 000 sphere nodes, 16.5 M bonds:
 // pre-pass 95 -> 56, main loop 78 -> 61.
 #include <cfloat>
 

@@ -216,7 +216,6 @@ struct DevData {
   int32_t contact_grid;  // blocks of the contact node pass
   Grid grid;
   int32_t *cell_of, *cell_cnt, *cell_start, *cell_fill, *cell_tmp, *cell_nodes;
-  unsigned long long bar_wait_ns;  // longest wait at a barrier of the contact rebuild
   // contact rebuild, per node in cell order: its particle and position
   int32_t *cell_p;
   double *cell_x;
@@ -325,6 +324,8 @@ struct DevData {
   int32_t n_tile_live_src;
   int32_t sur_interval;
   int32_t sur_near_gate;
+
+  unsigned long long bar_wait_ns;  // longest wait at a barrier of the contact rebuild
 };
 
 // ---- launchers (all asynchronous on `s`) ----
@@ -400,8 +401,9 @@ void launch_ctrl(const DevData &d, int mode, cudaStream_t s);  // mode 0 step, 1
 void launch_step_begin(const DevData &d, int verlet, cudaStream_t s);
 // external forces + force BC (+ Verlet second half) + post-processing (last CTA)
 void launch_step_end(const DevData &d, int verlet, int post, cudaStream_t s);
-// step end of one step and step begin of the next, in one kernel (scenes up
-// to kTurnMaxNodes nodes)
+// step end of one step and step begin of the next, in one kernel (scenes up to
+// kTurnMaxNodes nodes: 148 SMs x 4 CTAs x 256 threads, a wave of its CTAs in 2-D
+// and four thirds of one in 3-D, where three CTAs fit an SM)
 constexpr int64_t kTurnMaxNodes = 148 * 4 * 256;
 void launch_step_turn(const DevData &d, int verlet, cudaStream_t s);
 void launch_bc(const DevData &d, cudaStream_t s);

@@ -1235,7 +1235,7 @@ __global__ void __launch_bounds__(kBlock) k_contact(DevData d) {
 //
 // Particle-particle: one warp per particle, kBlock / 32 of them per CTA.  The
 // CTA stages the centres of kBlock particles at a time in FP32 and every warp
-// tests its particle against them with a 10 % margin over the largest reach
+// tests its particle against them with an 8 % margin over the largest reach
 // any zone pair allows (coordinates rounded to FP32 move a distance by far
 // less), so that only pairs the FP64 test can pass read FP64 data.
 //
@@ -2008,13 +2008,15 @@ __global__ void __launch_bounds__(kBlock) k_step_end(const __grid_constant__ Dev
 // the positions the post-processing needs go to d.turn before they move on;
 // the last CTA runs it, then the step control.
 //
-// For scenes up to a wave of CTAs (kTurnMaxNodes), where the two kernels are a
-// chain of latencies: us per step without / with it, two discs FP64 14.8 / 13.1,
-// PMB with Verlet 18.5 / 15.7, 24 000 nodes 26.4 / 24.9.  Larger ones gain
-// nothing (332 000 nodes 49.2 / 49.2 to 50.0, 1.3 M 154.1 / 152.8 to 158.7 over
-// one or two nodes per thread, bulk prefetch of later CTAs' nodes 156.5; 3-D,
-// 244 000 nodes 142.8 / 144.4): the traffic saved is a tenth, and the longer
-// kernel holds fewer warps.
+// For scenes up to about a wave of CTAs (kTurnMaxNodes), where the two kernels are
+// a chain of latencies: us per step without / with it, two discs FP64 14.8 / 13.1,
+// PMB with Verlet 18.5 / 15.7, 24 000 nodes 26.4 / 24.9, 151 000 nodes 32.5 / 28.8
+// (FP64 52.3 / 48.6); 3-D, 113 000 nodes 84.4 / 81.3, 147 000 nodes 56.4 / 54.7
+// (Verlet 96.5 / 93.3, FP64 114.8 / 112.6).  Larger ones gain nothing (332 000
+// nodes 49.2 / 49.2 to 50.0, 1.3 M 154.1 / 152.8 to 158.7 over one or two nodes
+// per thread, bulk prefetch of later CTAs' nodes 156.5; 3-D, 244 000 nodes
+// 142.8 / 144.4): the traffic saved is a tenth, and the longer kernel holds fewer
+// warps.
 // ---------------------------------------------------------------------------
 template <int DIM, bool VERLET>
 __global__ void __launch_bounds__(kBlock) k_step_turn(const __grid_constant__ DevData d) {

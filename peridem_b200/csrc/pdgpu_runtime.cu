@@ -665,11 +665,15 @@ int setup_tile_list(pdgpu_ctx *ctx) {
 // the CTA, two in the 2-D FP64 form (us per launch, FP64: 2-D, 333 000 nodes,
 // 84 at 4 lanes, 99 at 8; tile of 128 / 256 nodes 84 / 88; 3-D, 75 000 sphere
 // nodes, 73 at 4 lanes, 77 at 8; FP32 form, 3-D, 200 000 sphere nodes: tile of
-// 96 / 128 / 192 nodes 81 / 76 / 94).  The FP64 form raises the lanes of a
+// 96 / 128 / 192 nodes 81 / 76 / 94; 2-D, horizon of five mesh sizes, some 70 bonds
+// per node, four lanes, us per step, tile of 32 / 64 / 128 nodes: 24 000 nodes 23.7 /
+// 28.4 / 30.4, 135 000 40.3 / 44.6 / 46.9, 333 000 77.2 / 74.8 / 77.8).  The FP64
+// form raises the lanes of a
 // scene whose tiles would leave SMs idle, to the most whose one-pass tiles
 // still fit the chip at once (a pair, 317 nodes: bond loop 21 us at 8 lanes
-// and 128-node tiles, 4.8 us at 16 and 16).  The FP32 form keeps its lanes: its
-// partial sums are FP32, so their order shows in the results.
+// and 128-node tiles, 4.8 us at 16 and 16); the order of a node's FP64 sum thus
+// follows the size of its scene.  The FP32 form keeps its lanes: its partial
+// sums are FP32, so their order shows in the results.
 void choose_tiling(pdgpu_ctx *ctx) {
   const DevData &d = ctx->d;
   const bool mixed = d.precision == PDGPU_PREC_MIXED;
