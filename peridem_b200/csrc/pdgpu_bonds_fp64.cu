@@ -164,6 +164,8 @@ struct Bond64 {
   }
 };
 
+__device__ __forceinline__ bool not_finite(double a) { return (__double2hiint(a) & 0x7ff00000) == 0x7ff00000; }
+
 template <int LPN>
 __device__ __forceinline__ double gmax64(double v, int lanes) {
 #pragma unroll
@@ -404,7 +406,10 @@ __global__ void __launch_bounds__(kThreads64<DIM>, DIM == 2 ? 4 : 1)
     s.zmax = gmax64<LPN>(s.zmax, lpn);
     test |= may_break && !(s.zmax <= break_z);
     // a stretch that overflowed leaves its lane's force not a number
-    if constexpr (!PRE) test |= !(fabs(s.f[0]) + fabs(s.f[1]) + fabs(s.f[2]) <= DBL_MAX);
+    if constexpr (!PRE) {
+#pragma unroll
+      for (int q = 0; q < DIM; q++) test |= not_finite(s.f[q]);
+    }
     if (__any_sync(kFullWarp, test)) {
       if (test) {
         s = Sum64{};
